@@ -393,7 +393,8 @@ __global__ void k_mark(lgb_geom g, int np, const int *__restrict__ cell, const i
 /* Queued patches into the work-list region of their size class (cls_off); nwork counts them all.
    The cells around a queued patch node (up to 2^dim) are marked for a record rebuild. */
 __global__ void k_compact(lgb_geom g, int *__restrict__ need, const int *__restrict__ pm,
-                          const int *__restrict__ cls_off, int *__restrict__ work, lgb_ctrl *ctrl,
+                          const int *__restrict__ cls_off, int *__restrict__ work, int *__restrict__ work_s,
+                          const int *__restrict__ kept, unsigned blk, lgb_ctrl *ctrl,
                           unsigned char *__restrict__ cdirty)
 {
   int node = blockIdx.x * blockDim.x + threadIdx.x;
@@ -401,7 +402,9 @@ __global__ void k_compact(lgb_geom g, int *__restrict__ need, const int *__restr
   if (need[node]) {
     need[node] = 0;
     const int c = lgb_patch_class(pm[node]);
-    work[cls_off[c] + atomicAdd(&ctrl->nwork_c[c], 1)] = node;
+    /* kept: the set-up flags when factors are kept; blk: classes with a separate re-solve launch */
+    if (kept && kept[node] && ((blk >> c) & 1)) work_s[cls_off[c] + atomicAdd(&ctrl->nwork_s[c], 1)] = node;
+    else work[cls_off[c] + atomicAdd(&ctrl->nwork_c[c], 1)] = node;
     atomicAdd(&ctrl->nwork, 1);
     const int i = node % g.n[0], j = (node / g.n[0]) % g.n[1], k = node / (g.n[0] * g.n[1]);
     for (int dk = (g.dim == 3) ? -1 : 0; dk <= 0; dk++)
@@ -426,7 +429,7 @@ extern "C" int lgb_op_mark_patches(lgb_dev *d, void *stream)
 {
   cudaStream_t s = (cudaStream_t)stream;
   cudaMemsetAsync(&d->ctrl->nwork, 0, sizeof(int), s);
-  cudaMemsetAsync(d->ctrl->nwork_c, 0, sizeof(int) * LGB_NCLS, s);
+  cudaMemsetAsync(d->ctrl->nwork_c, 0, 4 * sizeof(int) * LGB_NCLS, s); /* next_c, nwork_s, next_s follow it */
   if (d->setup_all) {
     k_mark_all<<<lgb_cdiv(d->g.nnodes, 256), 256, 0, s>>>(d->g.nnodes, d->setup, d->solved, d->need);
     lgb_count_launch(1);
@@ -434,8 +437,10 @@ extern "C" int lgb_op_mark_patches(lgb_dev *d, void *stream)
     k_mark<<<lgb_cdiv(d->np, 256), 256, 0, s>>>(d->g, d->np, d->cell_p, d->alive, d->setup, d->solved, d->need);
     lgb_count_launch(1);
   }
-  k_compact<<<lgb_cdiv(d->g.nnodes, 256), 256, 0, s>>>(d->g, d->need, d->pm, d->cls_off_dev, d->work, d->ctrl,
-                                                        d->cdirty);
+  unsigned blk = 0;
+  for (int c = 0; c < LGB_NCLS; c++) blk |= (d->cls_threads[c] == 0 ? 1u : 0u) << c;
+  k_compact<<<lgb_cdiv(d->g.nnodes, 256), 256, 0, s>>>(d->g, d->need, d->pm, d->cls_off_dev, d->work, d->work_s,
+                                                        d->keep_factors ? d->setup : NULL, blk, d->ctrl, d->cdirty);
   lgb_count_launch(1);
   LGB_CHECK_LAUNCH();
   return 0;

@@ -1,5 +1,5 @@
 /*
- * lgb_factor.cu -- batched per-patch collocation assembly, FP64 Cholesky and solve.
+ * lgb_factor.cu -- batched per-patch collocation assembly, Cholesky and solve in FP64 precision.
  *
  * Replaces the lazy patch set-up and solve of LagRBF_PartitionsSetUp (src/partitions/partition.c:
  * 384-478): PartitionAssembleRBFMatrix (partition_solve.c:47-95, partition_asmb_avx512.c:119-198),
@@ -8,23 +8,24 @@
  *
  * Patches are queued by size class (LGB_NCLS classes of sizes up to 32, 64, ..., 2048 and beyond);
  * each class is one launch of a persistent grid over its work list (graph-capturable with a
- * device-side count), with the class's CTA size from the measured table (lgb_factor_tune.h), its
- * own workspace slot size (the class's largest patch) and as many CTAs as fit 1024 threads per SM
- * within the workspace budget.  The patch matrix is
- * assembled column-major into a per-CTA workspace slot (lower triangle), factored in panels of
- * CHOL_NB columns (left-looking inside a panel, then a tiled update of the trailing triangle), then
- * the F right-hand sides are solved together.  FP64 throughout: the collocation systems are
- * ill-conditioned.  A
- * non-positive pivot sets ctrl->factor_error (1-based row) and leaves the patch not set up; no
- * trap, no abort.  The factor is then "prepared" for the solves (reciprocal diagonal and scaled
- * diagonal blocks, below); when factors are kept (A_FACTOR / A_KSP) it is packed (column-major
- * lower, m(m+1)/2) so that new field values only need the two triangular solves, which run the same
- * code on the same values as the first solve.
+ * device-side count).  Patches of up to 64 points run k_factor<NT> (CTA size from the measured table
+ * lgb_factor_tune.h): the matrix is assembled column-major into a per-CTA workspace slot, factored in
+ * FP64 in panels of CHOL_NB columns, and solved.  Larger patches run k_factor_blk, whose updates are
+ * formed on the tensor cores and the integer pipe (below), and k_solve_blk where only the field values
+ * changed and the factor is kept (A_FACTOR / A_KSP).  The collocation systems are ill-conditioned: the
+ * error of the coefficients against extended precision is that of an FP64 factorisation or smaller
+ * (0.5-1.0 of it over patches of 196-343 points and kappa up to 1e9).  A non-positive pivot sets
+ * ctrl->factor_error (1-based row) and leaves the patch not set up; no trap, no abort.  Factors are
+ * "prepared" for the solves (reciprocal diagonal and scaled diagonal blocks, below); the first solve
+ * and re-solves run the same code on the same values.
  *
- * Roofline: FP64 pipe (m^3/3 flops per patch to factor, 2 F m^2 per solve); GB300 issues 2 DFMA
- * per clock per SM, so FP64 instructions, not bytes, are what the code counts.
+ * Roofline: GB300 issues 2 DFMA per clock per SM, which bounds an FP64 factorisation at m^3 / 6 / 2
+ * clocks per patch.  Measured: 1,728 patches of up to 729 points 148.9 ms in FP64 throughout, 24.9 ms
+ * with k_factor_blk (bound by the tensor cores' 21 digit products, then by the latency of the pivots);
+ * re-solve of 4,096 patches with kept factors 7.7 ms, then 3.7 ms (bound by reading the factor).
  */
 #include "lgb_common.cuh"
+#include "lgb_fx.cuh"
 
 #define CHOL_NB 16 /* columns per Cholesky panel */
 
@@ -41,6 +42,7 @@ struct FactorParams {
   float *c32;
   long long ws_stride;
   lgb_ctrl *ctrl;
+  int fixed;       /* blocked kernel: kernel values in fixed point (Wendland C2 of moderate extent) */
   double *kappa;   /* non-NULL: 1-norm condition estimate of every factored patch, by node */
 };
 
@@ -243,13 +245,13 @@ __device__ double blk_argmax_abs(const double *z, int m, int *idx, double *red, 
    N. J. Higham, "FORTRAN codes for estimating the one-norm of a real or complex matrix", ACM TOMS 14
    (1988); A symmetric, so A^-T = A^-1): at most five iterations of x -> sign(A^-1 x) -> e_j, then
    the alternating test vector x_i = (-1)^i (1 + i/(m-1)).  v, u: two workspace vectors of m. */
-__device__ double inv_norm1_estimate(const double *L, int m, double *v, double *u, double *D, double *Y, double *red,
-                                     int *ired)
+template <typename Solve>
+__device__ double inv_norm1_estimate(int m, double *v, double *u, double *red, int *ired, Solve solve)
 {
   const int tid = threadIdx.x;
   for (int i = tid; i < m; i += blockDim.x) v[i] = 1.0 / m;
   __syncthreads();
-  chol_solve_group<false, 1>(L, m, v, D, Y);
+  solve(v);
   double s = 0.0;
   for (int i = tid; i < m; i += blockDim.x) s += fabs(v[i]);
   double est = blk_reduce(s, red, false);
@@ -257,7 +259,7 @@ __device__ double inv_norm1_estimate(const double *L, int m, double *v, double *
   for (int it = 0; it < 5; it++) {
     for (int i = tid; i < m; i += blockDim.x) u[i] = (v[i] >= 0.0) ? 1.0 : -1.0;
     __syncthreads();
-    chol_solve_group<false, 1>(L, m, u, D, Y);
+    solve(u);
     int j;
     const double zmax = blk_argmax_abs(u, m, &j, red, ired);
     double ztx;
@@ -271,7 +273,7 @@ __device__ double inv_norm1_estimate(const double *L, int m, double *v, double *
     if (it > 0 && zmax <= ztx) break;
     for (int i = tid; i < m; i += blockDim.x) v[i] = (i == j) ? 1.0 : 0.0;
     __syncthreads();
-    chol_solve_group<false, 1>(L, m, v, D, Y);
+    solve(v);
     s = 0.0;
     for (int i = tid; i < m; i += blockDim.x) s += fabs(v[i]);
     const double e2 = blk_reduce(s, red, false);
@@ -281,18 +283,78 @@ __device__ double inv_norm1_estimate(const double *L, int m, double *v, double *
   }
   for (int i = tid; i < m; i += blockDim.x) v[i] = ((i & 1) ? -1.0 : 1.0) * (1.0 + (m > 1 ? (double)i / (m - 1) : 0.0));
   __syncthreads();
-  chol_solve_group<false, 1>(L, m, v, D, Y);
+  solve(v);
   s = 0.0;
   for (int i = tid; i < m; i += blockDim.x) s += fabs(v[i]);
   const double alt = 2.0 * blk_reduce(s, red, false) / (3.0 * m);
   return fmax(est, alt);
 }
 
-/* One template per CTA size NT (the patch-size class's entry of the tuning table). */
+/* The adjacent cells of a patch node (thread 0): first sorted point, count and offset in the patch. */
+struct PatchCells {
+  int cstart[8], cnt[8], off[8];
+};
+__device__ void patch_cells(const FactorParams &P, int node, PatchCells &C)
+{
+  const lgb_geom &g = P.g;
+  int nxy = g.n[0] * g.n[1];
+  int l = node / nxy, r = node - l * nxy, j = r / g.n[0], i = r - j * g.n[0];
+  for (int s = 0; s < 8; s++) {
+    int dx = s & 1, dy = (s >> 1) & 1, dz = (s >> 2) & 1;
+    int ci = i - 1 + dx, cj = j - 1 + dy, cl = (g.dim == 3) ? (l - 1 + dz) : 0;
+    bool ok = (g.dim == 3 || dz == 0) && ci >= 0 && ci < g.nc[0] && cj >= 0 && cj < g.nc[1] && cl >= 0 &&
+              cl < g.nc[2];
+    int c = ok ? ci + cj * g.nc[0] + cl * g.nc[0] * g.nc[1] : 0;
+    C.cstart[s] = ok ? P.cstart[c] : 0;
+    C.cnt[s] = ok ? P.cstart[c + 1] - P.cstart[c] : 0;
+    C.off[s] = P.slot[node * 8 + s];
+  }
+}
+
+/* The patch points (reference patch order) into X[m*dim] and their values into B[f*m + q]. */
+__device__ void patch_gather(const FactorParams &P, const PatchCells &C, int m, double *X, double *B)
+{
+  const int dim = P.g.dim;
+  for (int q = threadIdx.x; q < m; q += blockDim.x) {
+    int s = 0;
+    while (s < 7 && q >= C.off[s] + C.cnt[s]) s++;
+    int src = C.cstart[s] + (q - C.off[s]);
+    for (int d = 0; d < dim; d++) X[(size_t)q * dim + d] = P.xs[(size_t)src * dim + d];
+    for (int f = 0; f < P.F; f++) B[(size_t)f * m + q] = P.fs[(size_t)src * P.F + f];
+  }
+}
+
+/* The coefficients of a patch, [point][field], in both precisions, and its flags. */
+__device__ void patch_store(const FactorParams &P, int node, int m, const double *B)
+{
+  const int F = P.F;
+  const long long c0 = P.coff[node];
+  for (int q = threadIdx.x; q < m; q += blockDim.x)
+    for (int f = 0; f < F; f++) {
+      double v = B[(size_t)f * m + q];
+      P.c64[(size_t)(c0 + q) * F + f] = v;
+      P.c32[(size_t)(c0 + q) * F + f] = (float)v;
+    }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    P.setup[node] = 1;
+    P.solved[node] = 1;
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void count_factored(const FactorParams &P, int m)
+{
+  atomicAdd(&P.ctrl->factor_flops, (double)m * m * m / 3.0 + 2.0 * (double)m * m * P.F);
+  atomicAdd(&P.ctrl->nfactored, 1);
+}
+
+/* One template per CTA size NT (the patch-size class's entry of the tuning table): patches of up to 64
+   points, or every patch under the option factor_threads. */
 template <int NT>
 __global__ void __launch_bounds__(NT) k_factor(FactorParams P)
 {
-  __shared__ int s_cstart[8], s_cnt[8], s_off[8];
+  __shared__ PatchCells s_cells;
   __shared__ int s_fail;
   __shared__ double s_rd;
   __shared__ double s_diag[32 * 33], s_y[4 * 32];
@@ -307,31 +369,13 @@ __global__ void __launch_bounds__(NT) k_factor(FactorParams P)
     const int m = P.pm[node];
     const int F = P.F;
     if (tid == 0) {
-      int nxy = g.n[0] * g.n[1];
-      int l = node / nxy, r = node - l * nxy, j = r / g.n[0], i = r - j * g.n[0];
-      for (int s = 0; s < 8; s++) {
-        int dx = s & 1, dy = (s >> 1) & 1, dz = (s >> 2) & 1;
-        int ci = i - 1 + dx, cj = j - 1 + dy, cl = (g.dim == 3) ? (l - 1 + dz) : 0;
-        bool ok = (g.dim == 3 || dz == 0) && ci >= 0 && ci < g.nc[0] && cj >= 0 && cj < g.nc[1] && cl >= 0 &&
-                  cl < g.nc[2];
-        int c = ok ? ci + cj * g.nc[0] + cl * g.nc[0] * g.nc[1] : 0;
-        s_cstart[s] = ok ? P.cstart[c] : 0;
-        s_cnt[s] = ok ? P.cstart[c + 1] - P.cstart[c] : 0;
-        s_off[s] = P.slot[node * 8 + s];
-      }
+      patch_cells(P, node, s_cells);
       s_fail = 0;
     }
     __syncthreads();
     double *X = A + (size_t)m * m;     /* m*dim patch coordinates */
     double *B = X + (size_t)m * g.dim; /* m*F right-hand sides / solutions */
-    /* gather the patch points (reference patch order) and their values */
-    for (int q = tid; q < m; q += NT) {
-      int s = 0;
-      while (s < 7 && q >= s_off[s] + s_cnt[s]) s++;
-      int src = s_cstart[s] + (q - s_off[s]);
-      for (int d = 0; d < g.dim; d++) X[(size_t)q * g.dim + d] = P.xs[(size_t)src * g.dim + d];
-      for (int f = 0; f < F; f++) B[(size_t)f * m + q] = P.fs[(size_t)src * F + f];
-    }
+    patch_gather(P, s_cells, m, X, B);
     __syncthreads();
     const bool have_factor = P.setup[node] && P.keep;
     if (m > 0 && !have_factor) {
@@ -432,7 +476,9 @@ __global__ void __launch_bounds__(NT) k_factor(FactorParams P)
       if (s_fail) { __syncthreads(); continue; }
       prepare_diag_blocks<false>(A, m);
       if (P.kappa) {
-        const double inv = inv_norm1_estimate(A, m, Ps, Ps + m, s_diag, s_y, s_red, s_ired);
+        const double inv = inv_norm1_estimate(m, Ps, Ps + m, s_red, s_ired, [&](double *v) {
+          chol_solve_group<false, 1>(A, m, v, s_diag, s_y);
+        });
         if (tid == 0) P.kappa[node] = anorm * inv;
       }
       if (P.keep) {
@@ -442,10 +488,7 @@ __global__ void __launch_bounds__(NT) k_factor(FactorParams P)
           for (int i = j + tid; i < m; i += NT) Fk[base + (i - j)] = A[(size_t)j * m + i];
         }
       }
-      if (tid == 0) {
-        atomicAdd(&P.ctrl->factor_flops, (double)m * m * m / 3.0 + 2.0 * (double)m * m * F);
-        atomicAdd(&P.ctrl->nfactored, 1);
-      }
+      if (tid == 0) count_factored(P, m);
     } else if (m > 0) {
       if (tid == 0) atomicAdd(&P.ctrl->factor_flops, 2.0 * (double)m * m * F);
     }
@@ -453,21 +496,592 @@ __global__ void __launch_bounds__(NT) k_factor(FactorParams P)
     if (m > 0) {
       if (have_factor) chol_solve<true>(P.fac + P.foff[node], m, F, B, s_diag, s_y);
       else chol_solve<false>(A, m, F, B, s_diag, s_y);
-      /* coefficients [point][field] in both precisions */
-      const long long c0 = P.coff[node];
-      for (int q = tid; q < m; q += NT)
-        for (int f = 0; f < F; f++) {
-          double v = B[(size_t)f * m + q];
-          P.c64[(size_t)(c0 + q) * F + f] = v;
-          P.c32[(size_t)(c0 + q) * F + f] = (float)v;
+    }
+    patch_store(P, node, m, B);
+  }
+}
+
+/* ---- blocked factorisation with fixed-point updates -------------------------------------------- */
+/* GB300 issues 2 FP64 multiply-adds per clock and SM, so the updates of the factorisation (m^3 / 6
+   multiply-adds) run on the tensor cores and the integer pipe.  The kernels with a positive definite
+   matrix have phi(0) <= 1, so every factor entry l is in [-1, 1] and is held in fixed point, units of
+   2^-56 (lgb_fx.cuh), whose rounding is below that of FP64 from 1/8 on and below what the m rounded
+   FP64 subtractions of an entry accumulate:
+     - the sums over earlier block columns on the tensor cores: l = sum_i d_i 2^-(9 + 10 i) with six
+       balanced digits |d_i| <= 512, exact in FP16; the products of equal weight i + j <= 5 (21 of 36;
+       the others are below 2^-55 together) accumulate in FP32 and are moved to 64-bit integers every
+       64 columns.  Sums below 2^24 are exact: with row norms <= 1 (Cauchy) those with d_0 stay below
+       2^18 sqrt(64), sum d_1 d_1' <= 64 2^18, and sums of pairs of lower digits are of the order
+       sqrt(64) 2^16.4 (sums of squares on the diagonal 64 2^16.4);
+     - inside a block column as {hi, lo} integer multiply-adds (fx_mad), in 64-bit sums: |sum hi hi'|
+       <= 2^56, |sum hi lo' + lo hi'| <= 2^56 sqrt(32).
+   An entry beyond 1 proves a non-positive pivot in its row (a_ii - l_ij^2 < 0): it is clamped for the
+   updates and the row is remembered, so the factorisation stops there at the latest.
+
+   One CTA per patch, block columns of 32, left-looking.  For each block column the sums over all
+   earlier columns are formed in tiles of 64 rows (a warp: 16 rows x 16 columns, digit slabs of one
+   block column staged by cp.async) and subtracted from the kernel values, which are computed there and
+   never stored (Wendland C2 in fixed point, other kernels in FP64); the block column waits in the
+   workspace.  One warp factors the 32 x 32 diagonal block; then every thread solves its own rows
+   against it without further barriers.
+
+   The factor is stored by block columns of 32 columns x R_b = me - 32 b rows (me: m rounded up to
+   even, so that 16-byte copies of row pairs stay aligned): the diagonal block in FP64, prepared for
+   the solves as above, the rows below as {hi, lo}.  Fresh factors live in the workspace, kept ones in
+   the factor pool; the solves read the same format from either.  The digits live in the workspace. */
+#define BLK_NT 256
+#define BLK_NB 32
+#define BLK_KP 16   /* column pairs per staged slab (one block column) */
+#define BLK_ROWS 64
+#define BLK_ND 6    /* digits */
+#define BLK_FLUSH 2 /* slabs between two moves of the FP32 sums to integers */
+
+struct FxSolveShared {
+  int2 tile[128][36];   /* backward update: 128 columns x 32 rows, padded to distinct banks */
+  double d[32 * 33];    /* staged diagonal block */
+  int2 yq[4][32];       /* the block's solution in fixed point, relative to 2^e */
+  double ysc[4];        /* 2^(e - 56) */
+};
+struct FxFactorShared {
+  /* digit pairs (columns 2 p, 2 p + 1) of a row; row strides of 8 mod 32 words: the fragment reads of a
+     warp (four pairs x eight rows) fall in distinct banks */
+  union {
+    struct {
+      unsigned row[2][BLK_ND][BLK_KP][BLK_ROWS + 8];
+      unsigned col[2][BLK_ND][BLK_KP][BLK_NB + 8];
+    };
+    long long diag[BLK_NB][BLK_NB];  /* between the updates: the block's entries, [column][row] */
+  };
+  int2 q11[BLK_NB][BLK_NB];      /* diagonal block in fixed point, [row][column] */
+  double rd[BLK_NB];
+};
+struct BlkShared {
+  union {
+    FxSolveShared s;
+    FxFactorShared f;
+  };
+  double red[32];
+  PatchCells cells;
+  int ired[32];
+  int fail, badrow, item;
+};
+
+/* Start of block column b in the stored factor (8-byte elements) and in the digit array (words;
+   [digit][pair][row], rows from the block's first one, mh: m rounded up to a multiple of 4). */
+__device__ __forceinline__ long long fx_base(int me, int b) { return 32LL * b * me - 512LL * b * (b - 1); }
+__device__ __forceinline__ long long fx_dbase(int mh, int b) { return 16LL * BLK_ND * ((long long)b * mh - 16LL * b * (b - 1)); }
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, bool ok)
+{
+  const unsigned n = ok ? 16u : 0u; /* 0: zero fill */
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(n) : "memory");
+}
+
+/* Kernel value for the assembly from the squared distance (Wendland C2: lgb_sqrt_pos of (eps r)^2). */
+__device__ __forceinline__ double asm_phi(int kernel, double d2, double eps)
+{
+  if (kernel == LGB_KERNEL_WENDLAND_C2) {
+    const double s = d2 * (eps * eps);
+    const double r = lgb_sqrt_pos(s);
+    double u = 1.0 - r;
+    if (__double2hiint(u) < 0) return 0.0; /* the sign bit: no FP64 comparison */
+    const double u2 = u * u;
+    return (u2 * u2) * fma(-4.0, u, 5.0);
+  }
+  return lgb_phi<double>(kernel, sqrt(d2), eps);
+}
+
+/* Entry (i, j) of the collocation matrix in fixed point; X: the patch coordinates, FP64 or (fixed)
+   eps (x - node) in fixed point. */
+template <bool FIXED>
+__device__ __forceinline__ long long asm_entry(const lgb_geom &g, const double *X, int i, int j)
+{
+  if constexpr (FIXED) {
+    const long long *Z = reinterpret_cast<const long long *>(X);
+    long long s;
+    if (g.dim == 3)
+      s = fx_dist2<3>(Z[3 * (size_t)i] - Z[3 * (size_t)j], Z[3 * (size_t)i + 1] - Z[3 * (size_t)j + 1],
+                      Z[3 * (size_t)i + 2] - Z[3 * (size_t)j + 2]);
+    else s = fx_dist2<2>(Z[2 * (size_t)i] - Z[2 * (size_t)j], Z[2 * (size_t)i + 1] - Z[2 * (size_t)j + 1], 0);
+    return s < FX_ONE_I ? fx_phi_c2(s) : 0;
+  } else {
+    const int dim = g.dim;
+    const double *xi = X + (size_t)i * dim, *xj = X + (size_t)j * dim;
+    const double dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = (dim == 3) ? xi[2] - xj[2] : 0.0;
+    const double d2 = (dim == 3) ? fma(dx, dx, fma(dy, dy, dz * dz)) : fma(dx, dx, dy * dy);
+    return __double2ll_rn(asm_phi(g.kernel, d2, g.eps_r) * FX_ONE);
+  }
+}
+
+/* The balanced digits of two fixed-point values as FP16 pairs. */
+__device__ __forceinline__ void fx_digits(long long a, long long b, unsigned (&h)[BLK_ND])
+{
+  long long v[2] = {a << 3, b << 3}; /* units of 2^-59 */
+  float d[2][BLK_ND];
+#pragma unroll
+  for (int s = 0; s < 2; s++) {
+    long long t = v[s];
+#pragma unroll
+    for (int i = BLK_ND - 1; i > 0; i--) {
+      const int e = (int)((unsigned)t << 22) >> 22; /* the low ten bits, signed */
+      d[s][i] = (float)e;
+      t = (t - e) >> 10;
+    }
+    d[s][0] = (float)(int)t;
+  }
+#pragma unroll
+  for (int i = 0; i < BLK_ND; i++)
+    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(h[i]) : "f"(d[1][i]), "f"(d[0][i]));
+}
+
+__device__ __forceinline__ void blk_mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1)
+{
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+/* The block solution v (lane's entry, zero beyond the block) of right-hand side q into fixed point
+   relative to a power of two above its largest entry (one warp).  A solution that is not finite makes
+   every row it updates NaN through the scale. */
+__device__ __forceinline__ void fx_pack(FxSolveShared &S, int q, int lane, double v)
+{
+  const unsigned top = __reduce_max_sync(0xffffffffu, (unsigned)__double2hiint(v) & 0x7fffffffu) >> 20;
+  const int e = max((int)top - 1022, -900); /* |v| < 2^e */
+  const double up = __hiloint2double((1023 + 56 - e) << 20, 0);
+  S.yq[q][lane] = fx_split(top == 2047 ? 0 : __double2ll_rn(v * up));
+  if (lane == 0) S.ysc[q] = top == 2047 ? __hiloint2double(0x7ff80000, 0) : __hiloint2double((1023 - 56 + e) << 20, 0);
+}
+
+/* Solves L L^T X = B in place for FC (1..4) columns of B (B[q*m + i]) with the stored factor Fq, in
+   blocks of 32 rows: the diagonal block is substituted in FP64 (as chol_solve_group; one warp per
+   right-hand side, a warp issues an FP64 operation in 64 cycles), the other rows are updated with exact integer sums over the block and one FP64 multiply-add.  Forward:
+   a thread per row, coalesced along the rows.  Backward: tiles of 128 columns x 32 rows pass through
+   shared memory, two threads per column.  Bound by reading the factor (8 bytes per 9 integer
+   multiply-adds with three right-hand sides). */
+template <int FC>
+__device__ void fx_solve_group(const double *__restrict__ Fq, int m, double *B0, FxSolveShared &S)
+{
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nblk = (m + 31) / 32, me = (m + 1) & ~1;
+  for (int b = 0; b < nblk; b++) {
+    const int J = 32 * b, nb = min(32, m - J), R = me - J;
+    const double *Fb = Fq + fx_base(me, b);
+    for (int t = tid; t < 1024; t += BLK_NT) {
+      const int c = t >> 5, r = t & 31;
+      if (r >= c && r < nb) S.d[r * 33 + c] = Fb[(size_t)c * R + r];
+    }
+    __syncthreads();
+    if (warp < FC) {
+      double u = (lane < nb) ? B0[(size_t)warp * m + J + lane] : 0.0;
+      for (int jj = 0; jj < nb - 1; jj++) {
+        const double mij = (lane > jj && lane < nb) ? S.d[lane * 33 + jj] : 0.0;
+        u = fma(-mij, __shfl_sync(0xffffffffu, u, jj), u);
+      }
+      const double y = u * ((lane < nb) ? S.d[lane * 33 + lane] : 0.0);
+      if (lane < nb) B0[(size_t)warp * m + J + lane] = y;
+      fx_pack(S, warp, lane, lane < nb ? y : 0.0);
+    }
+    __syncthreads();
+    for (int i = J + 32 + tid; i < m; i += BLK_NT) {
+      const int2 *Lr = reinterpret_cast<const int2 *>(Fb) + (i - J);
+      long long hh[FC], hl[FC];
+#pragma unroll
+      for (int q = 0; q < FC; q++) { hh[q] = 0; hl[q] = 0; }
+#pragma unroll 16
+      for (int c = 0; c < 32; c++) {
+        const int2 l = Lr[(size_t)c * R];
+#pragma unroll
+        for (int q = 0; q < FC; q++) {
+          const int2 y = S.yq[q][c];
+          fx_mad(hh[q], l.x, y.x);
+          fx_mad(hl[q], l.x, y.y);
+          fx_mad(hl[q], l.y, y.x);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < FC; q++)
+        B0[(size_t)q * m + i] = fma(-(double)fx_sum(hh[q], hl[q]), S.ysc[q], B0[(size_t)q * m + i]);
+    }
+    __syncthreads();
+  }
+  for (int b = nblk - 1; b >= 0; b--) {
+    const int i0 = 32 * b, nb = min(32, m - i0), R = me - i0;
+    const double *Fb = Fq + fx_base(me, b);
+    for (int t = tid; t < 1024; t += BLK_NT) {
+      const int c = t >> 5, r = t & 31;
+      if (r >= c && r < nb) S.d[r * 33 + c] = Fb[(size_t)c * R + r];
+    }
+    __syncthreads();
+    if (warp < FC) {
+      double x = (lane < nb) ? B0[(size_t)warp * m + i0 + lane] * S.d[lane * 33 + lane] : 0.0;
+      for (int ii = nb - 1; ii >= 1; ii--) {
+        const double mi = (lane < ii) ? S.d[ii * 33 + lane] : 0.0;
+        x = fma(-mi, __shfl_sync(0xffffffffu, x, ii), x);
+      }
+      if (lane < nb) B0[(size_t)warp * m + i0 + lane] = x;
+      fx_pack(S, warp, lane, lane < nb ? x : 0.0);
+    }
+    __syncthreads();
+    for (int t0 = 0; t0 < i0; t0 += 128) {
+      for (int t = tid; t < 128 * 16; t += BLK_NT) {
+        const int c = t >> 4, i = t0 + c, bc = i >> 5;
+        if (i < i0)
+          cp_async16(&S.tile[c][2 * (t & 15)],
+                     Fq + fx_base(me, bc) + (size_t)(i & 31) * (me - 32 * bc) + (i0 - 32 * bc) + 2 * (t & 15), true);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();
+      const int c = tid >> 1, h = tid & 1, i = t0 + c;
+      long long hh[FC], hl[FC];
+#pragma unroll
+      for (int q = 0; q < FC; q++) { hh[q] = 0; hl[q] = 0; }
+      if (i < i0) {
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int r = 4 * k + 2 * h;
+          const int4 l = *reinterpret_cast<const int4 *>(&S.tile[c][r]);
+#pragma unroll
+          for (int q = 0; q < FC; q++) {
+            const int4 y = *reinterpret_cast<const int4 *>(&S.yq[q][r]);
+            fx_mad(hh[q], l.x, y.x);
+            fx_mad(hl[q], l.x, y.y);
+            fx_mad(hl[q], l.y, y.x);
+            fx_mad(hh[q], l.z, y.z);
+            fx_mad(hl[q], l.z, y.w);
+            fx_mad(hl[q], l.w, y.z);
+          }
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < FC; q++) {
+        hh[q] += __shfl_xor_sync(0xffffffffu, hh[q], 1);
+        hl[q] += __shfl_xor_sync(0xffffffffu, hl[q], 1);
+        if (h == 0 && i < i0)
+          B0[(size_t)q * m + i] = fma(-(double)fx_sum(hh[q], hl[q]), S.ysc[q], B0[(size_t)q * m + i]);
+      }
+      __syncthreads();
+    }
+    __syncthreads();
+  }
+}
+
+/* All F right-hand sides of B (B[f*m + i]), four at a time. */
+__device__ void fx_solve(const double *Fq, int m, int F, double *B, FxSolveShared &S)
+{
+  for (int f0 = 0; f0 < F; f0 += 4) {
+    double *B0 = B + (size_t)f0 * m;
+    switch (min(4, F - f0)) {
+    case 1: fx_solve_group<1>(Fq, m, B0, S); break;
+    case 2: fx_solve_group<2>(Fq, m, B0, S); break;
+    case 3: fx_solve_group<3>(Fq, m, B0, S); break;
+    default: fx_solve_group<4>(Fq, m, B0, S); break;
+    }
+  }
+}
+
+/* 1 / sqrt(d) of a double in the single range: the single-precision root y refined by a third-order
+   step (Householder's method); y^2 is exact in FP64, so the residual 1 - d y^2 is rounded once.  About
+   half an ulp in five operations.  (A warp issues an FP64 operation in 64 cycles, and this chain is
+   the pivot's latency.) */
+__device__ __forceinline__ double fx_rsqrt(double d)
+{
+  float f;
+  asm("rsqrt.approx.f32 %0, %1;" : "=f"(f) : "f"(__double2float_rn(d)));
+  const double y = (double)f, e = fma(-d, y * y, 1.0);
+  return fma(y * e, fma(e, 0.375, 0.5), y);
+}
+/* x 2^-56 for normal x (the exponent field: no FP64 operation). */
+__device__ __forceinline__ double fx_down(double x) { return __hiloint2double(__double2hiint(x) - (56 << 20), __double2loint(x)); }
+
+/* sum_k<N q[k] v[k] of the fixed-point entries, in CH (1 or 2) chains of integer sums. */
+template <int N, int CH>
+__device__ __forceinline__ long long fx_dot(const int2 (&q)[BLK_NB], const int2 *v)
+{
+  long long hh[CH], hl[CH];
+#pragma unroll
+  for (int c = 0; c < CH; c++) { hh[c] = 0; hl[c] = 0; }
+#pragma unroll
+  for (int k = 0; k < N; k++) {
+    const int2 x = v[k];
+    fx_mad(hh[k % CH], q[k].x, x.x);
+    fx_mad(hl[k % CH], q[k].x, x.y);
+    fx_mad(hl[(k + 1) % CH], q[k].y, x.x);
+  }
+  return CH == 2 ? fx_sum(hh[0] + hh[CH - 1], hl[0] + hl[CH - 1]) : fx_sum(hh[0], hl[0]);
+}
+
+/* One warp factors the nb x nb diagonal block J of the block column (lane i holds row J + i,
+   left-looking; S.diag: its entries): q11 and rd in shared memory, the prepared block in Fb.  Returns
+   the failing column + 1, or 0.  The chain of a column (dot product, pivot root, scaling) is the
+   latency of the factorisation. */
+template <int J0> struct BlkCol {
+  static __device__ __forceinline__ int run(FxFactorShared &S, int2 (&q)[BLK_NB], double *Fb, int J, int nb, int R, int lane,
+                                            int bad, int *badrow)
+  {
+    if (J0 >= nb) return 0;
+    const long long s = S.diag[J0][lane] - fx_dot<J0, 2>(q, S.q11[J0]);
+    const long long dd = __shfl_sync(0xffffffffu, s, J0);
+    if (dd <= 0 || J + J0 == bad) return J0 + 1;
+    const double rs = fx_rsqrt(fx_down((double)dd));
+    const double x = (double)s * rs;
+    long long f = __double2ll_rn(x); /* saturates */
+    if (f > FX_ONE_I + (1LL << 36) || f < -FX_ONE_I - (1LL << 36)) {
+      if (lane > J0 && lane < nb) atomicMin(badrow, J + lane);
+      f = f > 0 ? FX_ONE_I : -FX_ONE_I;
+    }
+    q[J0] = fx_split(f);
+    S.q11[lane][J0] = q[J0];
+    if (lane == J0) S.rd[J0] = rs;
+    if (lane >= J0 && lane < nb) Fb[(size_t)J0 * R + lane] = (J0 == lane) ? rs : x * fx_down(rs);
+    __syncwarp();
+    if constexpr (J0 + 1 < BLK_NB) return BlkCol<J0 + 1>::run(S, q, Fb, J, nb, R, lane, bad, badrow);
+    else return 0;
+  }
+};
+__device__ __noinline__ int blk_diag(FxFactorShared &S, double *Fb, int J, int nb, int R, int *badrow)
+{
+  int2 q[BLK_NB];
+  return BlkCol<0>::run(S, q, Fb, J, nb, R, threadIdx.x & 31, *badrow, badrow);
+}
+/* Block column J minus the sums over the columns before it, for the rows i0 .. i0 + 63 (all warps). */
+template <bool FIXED>
+__device__ __noinline__ void blk_update(FxFactorShared &T, const lgb_geom &g, const unsigned *H, const double *X,
+                                           long long *C, int m, int J, int i0)
+{
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, wr = warp & 3, wc = warp >> 2;
+  const int t = lane & 3, gr = lane >> 2, nslab = J / BLK_NB, mh = (m + 3) & ~3, rows = m - J;
+  float acc[BLK_ND][2][4]; /* by digit weight d + e */
+  long long v[2][4];
+#pragma unroll
+  for (int n = 0; n < 2; n++)
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      v[n][r] = 0;
+#pragma unroll
+      for (int s = 0; s < BLK_ND; s++) acc[s][n][r] = 0.f;
+    }
+  auto stage = [&](int sl) { /* block column sl: [digit][pair][row] */
+    const int bf = sl & 1, Rk = mh - 32 * sl;
+    const unsigned *src = H + fx_dbase(mh, sl);
+    {
+      const int c = 4 * (tid & 15), o = i0 - 32 * sl + c;
+      const bool ok = o < Rk;
+#pragma unroll
+      for (int d = 0; d < BLK_ND; d++)
+        cp_async16(&T.row[bf][d][tid >> 4][c], src + (size_t)(16 * d + (tid >> 4)) * Rk + (ok ? o : 0), ok);
+    }
+    {
+      const int c = 4 * (tid & 7), p = (tid >> 3) & 15, o = J - 32 * sl + c;
+      const bool ok = o < Rk;
+#pragma unroll
+      for (int d = 0; d < BLK_ND; d += 2)
+        cp_async16(&T.col[bf][d + (tid >> 7)][p][c], src + (size_t)(16 * (d + (tid >> 7)) + p) * Rk + (ok ? o : 0), ok);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  if (nslab > 0) stage(0);
+  for (int sl = 0; sl < nslab; sl++) {
+    if (sl + 1 < nslab) {
+      stage(sl + 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const int bf = sl & 1;
+#pragma unroll
+    for (int h = 0; h < BLK_KP; h += 8) {
+      unsigned a[BLK_ND][4];
+#pragma unroll
+      for (int d = 0; d < BLK_ND; d++) {
+        a[d][0] = T.row[bf][d][h + t][16 * wr + gr];
+        a[d][1] = T.row[bf][d][h + t][16 * wr + gr + 8];
+        a[d][2] = T.row[bf][d][h + t + 4][16 * wr + gr];
+        a[d][3] = T.row[bf][d][h + t + 4][16 * wr + gr + 8];
+      }
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int e = 0; e < BLK_ND; e++) {
+          const unsigned b0 = T.col[bf][e][h + t][16 * wc + 8 * n + gr], b1 = T.col[bf][e][h + t + 4][16 * wc + 8 * n + gr];
+#pragma unroll
+          for (int d = 0; d < BLK_ND; d++)
+            if (d + e < BLK_ND) blk_mma(acc[d + e][n], a[d], b0, b1);
+        }
+    }
+    if (sl % BLK_FLUSH == BLK_FLUSH - 1 || sl + 1 == nslab) {
+#pragma unroll
+      for (int n = 0; n < 2; n++)
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          long long x = (((long long)__float2int_rn(acc[4][n][r]) << 10) + __float2int_rn(acc[5][n][r]) + (1 << 11)) >> 12;
+#pragma unroll
+          for (int s = 0; s < 4; s++) x += (long long)__float2int_rn(acc[s][n][r]) << (38 - 10 * s);
+          v[n][r] += x;
+#pragma unroll
+          for (int s = 0; s < BLK_ND; s++) acc[s][n][r] = 0.f;
         }
     }
     __syncthreads();
+  }
+#pragma unroll
+  for (int n = 0; n < 2; n++)
+#pragma unroll
+    for (int r = 0; r < 4; r++) {
+      const int i = i0 + 16 * wr + gr + 8 * (r >> 1), jl = 16 * wc + 8 * n + 2 * t + (r & 1);
+      if (i >= m || i - J < jl) continue;
+      C[(size_t)jl * rows + (i - J)] = asm_entry<FIXED>(g, X, i, J + jl) - v[n][r];
+    }
+}
+
+/* Rows below the diagonal block: x L11^T = c, one row per thread, left to right; each entry's sum over
+   the columns before it in integers, one FP64 multiplication by the reciprocal pivot. */
+template <int J0> struct BlkRow {
+  static __device__ __forceinline__ bool run(const FxFactorShared &T, int2 (&q)[BLK_NB], const long long *C, int2 *Qb,
+                                             unsigned *Hb, int i, int rows, int R, int Rh, long long s, long long even)
+  {
+    long long ahead = 0;
+    if (J0 + 1 < BLK_NB) ahead = C[(size_t)(J0 + 1) * rows + i];
+    s -= fx_dot<J0, 1>(q, T.q11[J0]);
+    long long f = __double2ll_rn((double)s * T.rd[J0]); /* saturates */
+    bool bad = false;
+    if (f > FX_ONE_I + (1LL << 36) || f < -FX_ONE_I - (1LL << 36)) {
+      bad = true;
+      f = f > 0 ? FX_ONE_I : -FX_ONE_I;
+    }
+    q[J0] = fx_split(f);
+    Qb[(size_t)J0 * R + i] = q[J0];
+    if (J0 & 1) {
+      unsigned h[BLK_ND];
+      fx_digits(even, f, h);
+#pragma unroll
+      for (int d = 0; d < BLK_ND; d++) Hb[(size_t)(BLK_KP * d + (J0 >> 1)) * Rh + i] = h[d];
+    }
+    asm volatile("" ::: "memory"); /* one column's loads at a time: the row's entries fill the registers */
+    if constexpr (J0 + 1 < BLK_NB) bad |= BlkRow<J0 + 1>::run(T, q, C, Qb, Hb, i, rows, R, Rh, ahead, f);
+    return bad;
+  }
+};
+__device__ __noinline__ void blk_rows(BlkShared &S, const long long *C, int2 *Qb, unsigned *Hb, int J, int rows, int R, int Rh)
+{
+  for (int i = BLK_NB + threadIdx.x; i < rows; i += BLK_NT) {
+    int2 q[BLK_NB];
+    if (BlkRow<0>::run(S.f, q, C, Qb, Hb, i, rows, R, Rh, C[i], 0)) atomicMin(&S.badrow, J + i);
+  }
+}
+
+__global__ void __launch_bounds__(BLK_NT, 2) k_factor_blk(FactorParams P, int *next)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  BlkShared &S = *reinterpret_cast<BlkShared *>(smem_raw);
+  const lgb_geom &g = P.g;
+  const int nwork = *P.nwork, F = P.F, dim = g.dim;
+  const int tid = threadIdx.x, warp = tid >> 5;
+  double *W = P.ws + (size_t)blockIdx.x * P.ws_stride;
+  for (;;) {
+    if (tid == 0) S.item = atomicAdd(next, 1);
+    __syncthreads();
+    const int w = S.item;
+    if (w >= nwork) return;
+    const int node = P.work[w], m = P.pm[node], me = (m + 1) & ~1, mh = (m + 3) & ~3;
     if (tid == 0) {
-      P.setup[node] = 1;
-      P.solved[node] = 1;
+      patch_cells(P, node, S.cells);
+      S.fail = 0;
+      S.badrow = 0x7fffffff;
     }
     __syncthreads();
+    /* workspace: digits, block column, coordinates, right-hand sides, two vectors, then the factor */
+    unsigned *H = reinterpret_cast<unsigned *>(W);
+    long long *C = reinterpret_cast<long long *>(W + lgb_fx_dsize(m));
+    double *X = reinterpret_cast<double *>(C + (size_t)BLK_NB * m), *B = X + (size_t)m * dim, *V = B + (size_t)m * F;
+    double *Fq = P.keep ? P.fac + P.foff[node]
+                        : W + ((lgb_fx_dsize(m) + (long long)m * (BLK_NB + dim + F + 2) + 1) & ~1LL);
+    patch_gather(P, S.cells, m, X, B);
+    if (P.fixed) { /* coordinates relative to the patch node, scaled (each thread its own points) */
+      const int nxy = g.n[0] * g.n[1], l = node / nxy, r = node - l * nxy, nj = r / g.n[0];
+      const double c[3] = {g.O[0] + g.h[0] * (r - nj * g.n[0]), g.O[1] + g.h[1] * nj, g.O[2] + g.h[2] * l};
+      for (int q = tid; q < m; q += BLK_NT)
+        for (int d = 0; d < dim; d++) {
+          const long long z = fx_coord(g.eps_r, X[(size_t)q * dim + d] - c[d]);
+          X[(size_t)q * dim + d] = __longlong_as_double(z);
+        }
+    }
+    __syncthreads();
+    double anorm = 0.0;
+    if (P.kappa) { /* 1-norm of the symmetric matrix for the condition estimate */
+      double cm = 0.0;
+      for (int j = tid; j < m; j += BLK_NT) {
+        double cs = 0.0;
+        for (int i = 0; i < m; i++)
+          cs += fabs((double)(P.fixed ? asm_entry<true>(g, X, i, j) : asm_entry<false>(g, X, i, j)));
+        cm = fmax(cm, cs * (1.0 / FX_ONE));
+      }
+      anorm = blk_reduce(cm, S.red, true);
+    }
+    for (int J = 0; J < m; J += BLK_NB) {
+      const int nb = min(BLK_NB, m - J), rows = m - J, R = me - J, b = J / BLK_NB;
+      double *Fb = Fq + fx_base(me, b);
+      for (int i0 = J; i0 < m; i0 += BLK_ROWS) {
+        if (P.fixed) blk_update<true>(S.f, g, H, X, C, m, J, i0);
+        else blk_update<false>(S.f, g, H, X, C, m, J, i0);
+      }
+      __syncthreads();
+      for (int q = tid; q < BLK_NB * BLK_NB; q += BLK_NT) {
+        const int j = q / BLK_NB, r = q % BLK_NB;
+        S.f.diag[j][r] = (r >= j && r < nb) ? C[(size_t)j * rows + r] : 0;
+      }
+      __syncthreads();
+      if (warp == 0) {
+        const int failed = blk_diag(S.f, Fb, J, nb, R, &S.badrow);
+        if (failed && tid == 0) {
+          if (atomicCAS(&P.ctrl->factor_error, 0, J + failed) == 0) P.ctrl->factor_node = node;
+          S.fail = 1;
+        }
+      }
+      __syncthreads();
+      if (S.fail) break;
+      int2 *Qb = reinterpret_cast<int2 *>(Fb);
+      blk_rows(S, C, Qb, H + fx_dbase(mh, b), J, rows, R, mh - J);
+      if ((m & 1) && tid < BLK_NB) Qb[(size_t)tid * R + rows] = make_int2(0, 0); /* the padding row */
+      __syncthreads();
+    }
+    if (S.fail) continue; /* uniform: its write was followed by a barrier */
+    if (P.kappa) {
+      const double inv = inv_norm1_estimate(m, V, V + m, S.red, S.ired, [&](double *v) { fx_solve_group<1>(Fq, m, v, S.s); });
+      if (tid == 0) P.kappa[node] = anorm * inv;
+    }
+    if (tid == 0) count_factored(P, m);
+    fx_solve(Fq, m, F, B, S.s);
+    patch_store(P, node, m, B);
+  }
+}
+
+/* Re-solve of the patches with a kept factor of the blocked kernel. */
+__global__ void __launch_bounds__(BLK_NT) k_solve_blk(FactorParams P, int *next)
+{
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  FxSolveShared &S = *reinterpret_cast<FxSolveShared *>(smem_raw);
+  __shared__ PatchCells s_cells;
+  __shared__ int s_item;
+  const int nwork = *P.nwork, tid = threadIdx.x;
+  double *W = P.ws + (size_t)blockIdx.x * P.ws_stride;
+  for (;;) {
+    if (tid == 0) {
+      s_item = atomicAdd(next, 1);
+      if (s_item < nwork) patch_cells(P, P.work[s_item], s_cells);
+    }
+    __syncthreads();
+    if (s_item >= nwork) return;
+    const int node = P.work[s_item], m = P.pm[node];
+    double *X = W, *B = X + (size_t)m * P.g.dim;
+    patch_gather(P, s_cells, m, X, B);
+    if (tid == 0) atomicAdd(&P.ctrl->factor_flops, 2.0 * (double)m * m * P.F);
+    __syncthreads();
+    fx_solve(P.fac + P.foff[node], m, P.F, B, S);
+    patch_store(P, node, m, B);
   }
 }
 
@@ -495,6 +1109,10 @@ extern "C" int lgb_op_factor(lgb_dev *d, void *stream)
   P.ws_stride = d->ws_stride;
   P.ctrl = d->ctrl;
   P.kappa = d->cond_on ? d->kappa : NULL;
+  /* fixed-point coordinates eps (x - node) span |eps h|; 32 leaves the distances well inside 64 bits */
+  double ext = 0.0;
+  for (int i = 0; i < d->g.dim; i++) ext = fmax(ext, d->g.eps_r * d->g.h[i]);
+  P.fixed = d->g.kernel == LGB_KERNEL_WENDLAND_C2 && ext < 32.0;
   /* one launch per patch-size class holding patches: its CTA size, grid and workspace slots */
   for (int c = 0; c < LGB_NCLS; c++) {
     if (d->cls_cap[c] <= 0 || d->cls_grid[c] <= 0) continue;
@@ -503,6 +1121,24 @@ extern "C" int lgb_op_factor(lgb_dev *d, void *stream)
     P.ws_stride = d->cls_stride[c];
     cudaStream_t s = (cudaStream_t)stream;
     switch (d->cls_threads[c]) {
+    case 0: {
+      static int attr = 0; /* threads racing on it all set the same value */
+      if (!attr) {
+        cudaFuncSetAttribute(k_factor_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlkShared));
+        cudaFuncSetAttribute(k_solve_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSolveShared));
+        attr = 1;
+      }
+      k_factor_blk<<<d->cls_grid[c], BLK_NT, sizeof(BlkShared), s>>>(P, &d->ctrl->next_c[c]);
+      if (P.keep) {
+        FactorParams Q = P;
+        Q.work = d->work_s + d->cls_off[c];
+        Q.nwork = &d->ctrl->nwork_s[c];
+        Q.ws_stride = d->cls_sstride[c];
+        k_solve_blk<<<d->cls_sgrid[c], BLK_NT, sizeof(FxSolveShared), s>>>(Q, &d->ctrl->next_s[c]);
+        lgb_count_launch(1);
+      }
+      break;
+    }
     case 32: k_factor<32><<<d->cls_grid[c], 32, 0, s>>>(P); break;
     case 64: k_factor<64><<<d->cls_grid[c], 64, 0, s>>>(P); break;
     case 256: k_factor<256><<<d->cls_grid[c], 256, 0, s>>>(P); break;

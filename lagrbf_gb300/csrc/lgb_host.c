@@ -349,7 +349,7 @@ static void destroy_ctx(lgb_ctx *c)
   free_data(d);
   free_particles(d);
   DFREE(d->cstart); DFREE(d->dfill); DFREE(d->pm); DFREE(d->slot); DFREE(d->setup); DFREE(d->solved);
-  DFREE(d->need); DFREE(d->work); DFREE(d->status); DFREE(d->coff); DFREE(d->foff); DFREE(d->c64); DFREE(d->kappa);
+  DFREE(d->need); DFREE(d->work); DFREE(d->work_s); DFREE(d->status); DFREE(d->coff); DFREE(d->foff); DFREE(d->c64); DFREE(d->kappa);
   DFREE(d->c32); DFREE(d->fac); DFREE(d->ws); DFREE(d->pcount); DFREE(d->pstart); DFREE(d->pfill);
   DFREE(d->chunk_start); DFREE(d->scan_tmp); DFREE(d->scan_tmp64); DFREE(d->ctrl);
   DFREE(d->rec32); DFREE(d->rec_off); DFREE(d->bkey_buf); DFREE(d->cls_off_dev); DFREE(d->cdirty);
@@ -567,6 +567,7 @@ static int create_ctx(lgb_ctx **out)
   d->solved = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
   d->need = (int *)dalloc(sizeof(int) * 2 * (size_t)nn, &err);
   d->work = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
+  d->work_s = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
   d->status = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
   d->coff = (long long *)dalloc(sizeof(long long) * (size_t)(nn + 1), &err);
   d->foff = (long long *)dalloc(sizeof(long long) * (size_t)(nn + 1), &err);
@@ -695,7 +696,8 @@ static int grow_pids(int64_t **a, int *cap, int old_n, int n)
 }
 
 /* Patch-size classes of the set-up / solve launches: per class the work-list region (by the number
-   of its patches), the CTA size (option factor_threads, else the measured table), the workspace
+   of its patches), the CTA size (option factor_threads, else the blocked kernel or the measured
+   table), the workspace
    slot of its largest patch (m^2 + m (dim + F) + 17 m + 32 doubles: matrix, coordinates,
    right-hand sides, Cholesky panel rows) and a grid of 1024 / T CTAs per SM; the pool holds the
    largest class grid x slot, at most LGB_FACT_WS_BYTES (a class with bigger slots runs fewer CTAs). */
@@ -719,11 +721,20 @@ static int plan_classes(lgb_ctx *c)
   d->nws = 0;
   for (k = 0; k < LGB_NCLS; k++) {
     const long long m = cls_m[k] > 0 ? cls_m[k] : 1;
-    const int T = d->factor_threads ? d->factor_threads : lgb_factor_threads[k];
-    long long grid = (long long)(1024 / T) * d->nsm;
+    /* patches above 64 points: the blocked kernel (T = 0, two CTAs per SM, which also keeps the
+       factor in fixed point), and a separate launch for re-solves */
+    const int blk = !d->factor_threads && k >= LGB_FACT_BLK_CLS && m <= LGB_FACT_BLK_MAXM;
+    const int T = blk ? 0 : d->factor_threads ? d->factor_threads : lgb_factor_threads[k];
+    long long grid = (long long)(blk ? 2 : 1024 / T) * d->nsm;
     d->cls_off[k + 1] = d->cls_off[k] + d->cls_cap[k];
     d->cls_threads[k] = T;
-    d->cls_stride[k] = m * m + m * (d->g.dim + d->F) + m * 17 + 32;
+    d->cls_stride[k] = blk ? lgb_fx_dsize((int)m) + m * (32 + d->g.dim + d->F + 2) + 2 +
+                                 (d->keep_factors ? 0 : lgb_fx_size((int)m))
+                           : m * m + m * (d->g.dim + d->F) + m * 17 + 32;
+    d->cls_stride[k] += d->cls_stride[k] & 1; /* 16-byte aligned slots */
+    d->cls_sgrid[k] = 4 * d->nsm < d->cls_cap[k] ? 4 * d->nsm : d->cls_cap[k];
+    d->cls_sstride[k] = m * (d->g.dim + d->F) + 2;
+    if (blk && d->keep_factors && d->cls_sgrid[k] * d->cls_sstride[k] > pool) pool = d->cls_sgrid[k] * d->cls_sstride[k];
     if (grid > d->cls_cap[k]) grid = d->cls_cap[k];
     if (grid * d->cls_stride[k] * 8 > LGB_FACT_WS_BYTES) grid = LGB_FACT_WS_BYTES / (d->cls_stride[k] * 8);
     if (grid < 1 && d->cls_cap[k] > 0) grid = 1;
@@ -757,13 +768,18 @@ static int ensure_pools(lgb_ctx *c)
     d->c32 = (float *)dalloc(sizeof(float) * (size_t)d->coef_cap, &err);
     if (err) { d->coef_cap = 0; return set_error(LAGRBF_ERR_MEM, "coefficient pool allocation failed"); }
   }
+  TRY(plan_classes(c));
   if (d->keep_factors) {
-    /* packed factor offsets: exclusive scan of m(m+1)/2, computed on the host from pm */
+    /* offsets of the kept factors (even, for 16-byte copies), computed on the host from pm */
     int *pm = (int *)malloc(sizeof(int) * (size_t)nn), i;
     long long *fo = (long long *)malloc(sizeof(long long) * (size_t)(nn + 1));
     if (!pm || !fo) { free(pm); free(fo); return set_error(LAGRBF_ERR_MEM, "out of host memory"); }
     CUF(cudaMemcpy(pm, d->pm, sizeof(int) * (size_t)nn, cudaMemcpyDeviceToHost), (free(pm), free(fo)));
-    for (i = 0; i < nn; i++) { fo[i] = ftotal; ftotal += (long long)pm[i] * (pm[i] + 1) / 2; }
+    for (i = 0; i < nn; i++) {
+      fo[i] = ftotal;
+      ftotal += d->cls_threads[lgb_patch_class(pm[i])] == 0 ? lgb_fx_size(pm[i])
+                                                           : ((long long)pm[i] * (pm[i] + 1) / 2 + 1) & ~1LL;
+    }
     fo[nn] = ftotal;
     CUF(cudaMemcpy(d->foff, fo, sizeof(long long) * (size_t)(nn + 1), cudaMemcpyHostToDevice), (free(pm), free(fo)));
     free(pm); free(fo);
@@ -774,7 +790,6 @@ static int ensure_pools(lgb_ctx *c)
       if (err) { d->fac_cap = 0; return set_error(LAGRBF_ERR_MEM, "factor pool allocation failed (%lld doubles)", ftotal); }
     }
   }
-  TRY(plan_classes(c));
   return 0;
 }
 

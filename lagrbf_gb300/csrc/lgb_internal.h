@@ -49,6 +49,12 @@ enum { LGB_VF_NONE = 0, LGB_VF_ROTATION = 1, LGB_VF_CELLULAR = 2, LGB_VF_ABC = 3
    measured entry.  A class with CTAs of T threads keeps 1024 / T of them in flight per SM. */
 #define LGB_NCLS 8
 #define LGB_FACT_T 128
+/* First class of the blocked factorisation (cls_threads 0).  Set-up of every patch, blocked against
+   the best CTA size of the unblocked kernel: largest patch 39 points 2.01 / 1.86 ms (9,261 patches),
+   64 points 4.40 / 2.94 ms; 140 points 2.22-2.59 / 3.95 ms (2,197), 318 points 13.2 / 33.0 ms,
+   863 points 52.8 / 346 ms, 1,295 points 128 / 1249 ms. */
+#define LGB_FACT_BLK_CLS 2
+#define LGB_FACT_BLK_MAXM 16384 /* largest patch of its fixed-point sums */
 #ifdef __CUDACC__
 #define LGB_HD __host__ __device__
 #else
@@ -59,6 +65,18 @@ static inline LGB_HD int lgb_patch_class(int m)
   int c = 0;
   while (c < LGB_NCLS - 1 && m > (32 << c)) c++;
   return c;
+}
+/* 8-byte elements of the blocked kernel's stored factor of m points (layout in lgb_factor.cu). */
+static inline LGB_HD long long lgb_fx_size(int m)
+{
+  const long long me = (m + 1) & ~1, b = (m + 31) / 32;
+  return 32 * b * me - 512 * b * (b - 1);
+}
+/* Its digit array in the workspace, in 8-byte elements (even). */
+static inline LGB_HD long long lgb_fx_dsize(int m)
+{
+  const long long mh = (m + 3) & ~3, b = (m + 31) / 32;
+  return 48 * (b * mh - 16 * b * (b - 1)); /* six digits, 16 column pairs, 4 bytes */
 }
 /* FP32 record of one data point as the gather kernel stages it in shared memory: a header {x, x, y,
    y, z, z, 0, 0} (coordinates relative to the evaluating cell's origin, each twice so that one
@@ -116,6 +134,8 @@ typedef struct {
   int nfactored;
   double factor_flops;
   int nwork_c[LGB_NCLS];  /* queued patches of each size class (the class work lists)      */
+  int next_c[LGB_NCLS];   /* next entry of each class's work list (blocked factorisation)  */
+  int nwork_s[LGB_NCLS], next_s[LGB_NCLS]; /* the same of the patches that only re-solve        */
   int eval_error;      /* a bounded wait of the evaluation kernel gave up */
   int pp_left;         /* per-particle Dormand-Prince: particles still short of t_next   */
   double dt_cfl_ext;   /* > 0: the CFL step agreed over ranks (replaces the local one)     */
@@ -137,7 +157,7 @@ typedef struct {
   int *cell_d, *cstart, *sorted, *dfill, *dtmp;
   int max_cell_pts;
   /* patches */
-  int *pm, *slot, *setup, *solved, *work, *status;
+  int *pm, *slot, *setup, *solved, *work, *work_s, *status;
   int *need;          /* 2*nnodes ints: flags, also borrowed as nnodes int64 scratch */
   long long *coff, *foff;
   long long coef_cap, fac_cap;
@@ -160,6 +180,8 @@ typedef struct {
      and workspace slot stride (doubles) of each class launch; cls_off_dev on the device */
   int cls_off[LGB_NCLS + 1], cls_cap[LGB_NCLS], cls_threads[LGB_NCLS], cls_grid[LGB_NCLS];
   long long cls_stride[LGB_NCLS];
+  int cls_sgrid[LGB_NCLS];          /* re-solve launches of the blocked classes (work_s)     */
+  long long cls_sstride[LGB_NCLS];
   int *cls_off_dev;
   int factor_threads;  /* option factor_threads: one CTA size for every class (0: the table) */
   /* particle swarm */
