@@ -15,6 +15,7 @@
  * gives the offset of adjacent cell s inside the patch.
  */
 #include "lgb_common.cuh"
+#include "lgb_fx.cuh"
 #include <limits.h>
 
 static long long g_launches = 0;
@@ -221,7 +222,7 @@ __global__ void k_segsort(int ncells, const int *__restrict__ start, int *__rest
 /* ------------------------------------------------------------------------------------------- */
 __global__ void k_gather_data(lgb_geom g, int nd, int F, const int *__restrict__ sorted, const int *__restrict__ cell,
                               const double *__restrict__ xd, const double *__restrict__ fd, double *__restrict__ xs,
-                              float *__restrict__ xr, double *__restrict__ fs)
+                              float *__restrict__ xr, double *__restrict__ fs, long long *__restrict__ xq)
 {
   int s = blockIdx.x * blockDim.x + threadIdx.x;
   if (s >= nd) return;
@@ -236,6 +237,7 @@ __global__ void k_gather_data(lgb_geom g, int nd, int F, const int *__restrict__
     if (xs) xs[(size_t)s * g.dim + d] = v;
     /* coordinate relative to the origin node of the point's own cell */
     r[d] = (float)(v - (g.O[d] + g.h[d] * cc[d]));
+    if (xq) xq[(size_t)s * g.dim + d] = fx_coord(g.eps_r, v - (g.O[d] + g.h[d] * cc[d]));
   }
   if (xr) reinterpret_cast<float4 *>(xr)[s] = make_float4(r[0], r[1], r[2], 0.f);
   if (fs)
@@ -288,7 +290,7 @@ extern "C" int lgb_op_data_arrange(lgb_dev *d, void *stream)
   if ((rc = lgb_op_scatter(nd, d->cell_d, NULL, d->cstart, d->dfill, d->sorted, stream))) return rc;
   k_segsort<<<g.ncells, 256, 0, s>>>(g.ncells, d->cstart, d->sorted, d->dtmp);
   k_gather_data<<<lgb_cdiv(nd > 0 ? nd : 1, 256), 256, 0, s>>>(g, nd, d->F, d->sorted, d->cell_d, d->xd, d->fd,
-                                                                d->xs, d->xr, d->fs);
+                                                                d->xs, d->xr, d->fs, d->fixed ? d->xq : NULL);
   lgb_count_launch(2);
   LGB_CHECK_LAUNCH();
   /* patch sizes -> coefficient pool offsets */

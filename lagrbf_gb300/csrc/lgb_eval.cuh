@@ -59,6 +59,8 @@ struct EvalParams {
   const long long *rec_off;
   int poll_limit;         /* polls of a bounded mbarrier wait before it gives up          */
   int withhold_copies;    /* test hook: arm the staging barriers but issue no copy         */
+  const long long *xq;    /* [nd*dim] eps (x - own cell's origin) in fixed point, cell order */
+  const int *cexp;        /* [nnodes*F] exponents above the patches' coefficients             */
   unsigned char *cdirty;  /* cells whose record blocks must be rebuilt (set by the work-list compaction) */
 };
 
@@ -95,6 +97,14 @@ __host__ __device__ constexpr int eslot(int dim, int k, int o)
   return (eoff_a(o) - ecorner_ox(k) + 1) + 2 * (eoff_b(o) - ecorner_oy(k) + 1) +
          (dim == 3 ? 4 * (eoff_e(dim, o) - ecorner_oz(dim, k) + 1) : 0);
 }
+/* Virtual segments: the neighbour offsets, in 3D with the centre cell (in all eight corner patches)
+   twice, for corners 0-3 and 4-7, so that a segment involves at most four patches. */
+__host__ __device__ constexpr int vs_off(int dim, int vs) { return (dim == 3 && vs > 13) ? vs - 1 : vs; }
+__host__ __device__ constexpr int vs_mask(int dim, int vs)
+{
+  return einv_mask(dim, vs_off(dim, vs)) & ((dim == 3 && vs == 13) ? 0x0F : (dim == 3 && vs == 14) ? 0xF0 : 0xFF);
+}
+template <int DIM> struct VGeo { static constexpr int NVS = LGB_NVSEG(DIM); };
 /* Record length (elements) for a neighbour offset: 4 coordinates + ninv*FP coefficients, padded
    to a 16-byte multiple. */
 template <typename Real> __host__ __device__ constexpr int erec(int ninv, int fp)

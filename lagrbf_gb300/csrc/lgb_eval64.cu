@@ -8,6 +8,7 @@
 
 extern "C" int lgb_eval32_launch_3d(const EvalParams *P, int fp, int ker, int stage, int grid, void *stream);
 extern "C" int lgb_eval32_launch_2d(const EvalParams *P, int fp, int ker, int stage, int grid, void *stream);
+extern "C" int lgb_evalfx_launch(const EvalParams *P, int fp, int grid, void *stream);
 extern "C" int lgb_build_records_3d(const EvalParams *P, int force, int grid, void *stream);
 extern "C" int lgb_build_records_2d(const EvalParams *P, int force, int grid, void *stream);
 
@@ -93,12 +94,16 @@ extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int ou
     P.rec_off = d->rec_off;
     P.poll_limit = d->eval_poll_limit > 0 ? d->eval_poll_limit : EVAL_POLL_LIMIT;
     P.withhold_copies = d->eval_withhold;
+    P.xq = d->xq;
+    P.cexp = d->cexp;
     int rc;
     if (d->prec == LGB_PREC_FP32) {
       const int stage = (d->rec32 && f == 0 && fp == g.dim && d->rec_fp == g.dim) ? 1 : 0;
       P.budget = stage ? tma_budget() : BUDGET32;
       rc = (g.dim == 3) ? lgb_eval32_launch_3d(&P, fp, ker, stage, grid, stream)
                         : lgb_eval32_launch_2d(&P, fp, ker, stage, grid, stream);
+    } else if (d->fixed) {
+      rc = lgb_evalfx_launch(&P, fp, grid, stream);
     } else {
       P.budget = BUDGET64;
       rc = (g.dim == 3) ? launch64_fp<3>(P, fp, grid, s) : launch64_fp<2>(P, fp, grid, s);

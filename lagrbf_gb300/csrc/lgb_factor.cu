@@ -40,9 +40,10 @@ struct FactorParams {
   int *setup, *solved;
   double *c64, *fac, *ws;
   float *c32;
+  int *cexp;
   long long ws_stride;
   lgb_ctrl *ctrl;
-  int fixed;       /* blocked kernel: kernel values in fixed point (Wendland C2 of moderate extent) */
+  int fixed;       /* blocked kernel: kernel values in fixed point */
   double *kappa;   /* non-NULL: 1-norm condition estimate of every factored patch, by node */
 };
 
@@ -335,6 +336,22 @@ __device__ void patch_store(const FactorParams &P, int node, int m, const double
       P.c64[(size_t)(c0 + q) * F + f] = v;
       P.c32[(size_t)(c0 + q) * F + f] = (float)v;
     }
+  /* the fields' exponents, for the fixed-point evaluation */
+  __shared__ unsigned s_top;
+  for (int f = 0; f < F; f++) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_top = 0;
+    __syncthreads();
+    unsigned top = 0;
+    for (int q = threadIdx.x; q < m; q += blockDim.x) top = max(top, (unsigned)__double2hiint(B[(size_t)f * m + q]) & 0x7fffffffu);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) atomicMax(&s_top, top);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      const int e = (int)(s_top >> 20);
+      P.cexp[(size_t)node * F + f] = e == 2047 ? LGB_CEXP_NAN : e - 1022;
+    }
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
     P.setup[node] = 1;
@@ -592,19 +609,22 @@ __device__ __forceinline__ double asm_phi(int kernel, double d2, double eps)
   return lgb_phi<double>(kernel, sqrt(d2), eps);
 }
 
-/* Entry (i, j) of the collocation matrix in fixed point; X: the patch coordinates, FP64 or (fixed)
-   eps (x - node) in fixed point. */
-template <bool FIXED>
+/* Entry (i, j) of the collocation matrix in fixed point; X: the patch coordinates, FP64 (FIXED 0) or
+   eps (x - node) in fixed point (1: Wendland C2, 2: Gaussian). */
+template <int FIXED>
 __device__ __forceinline__ long long asm_entry(const lgb_geom &g, const double *X, int i, int j)
 {
-  if constexpr (FIXED) {
+  if constexpr (FIXED != 0) {
     const long long *Z = reinterpret_cast<const long long *>(X);
-    long long s;
-    if (g.dim == 3)
-      s = fx_dist2<3>(Z[3 * (size_t)i] - Z[3 * (size_t)j], Z[3 * (size_t)i + 1] - Z[3 * (size_t)j + 1],
-                      Z[3 * (size_t)i + 2] - Z[3 * (size_t)j + 2]);
-    else s = fx_dist2<2>(Z[2 * (size_t)i] - Z[2 * (size_t)j], Z[2 * (size_t)i + 1] - Z[2 * (size_t)j + 1], 0);
-    return s < FX_ONE_I ? fx_phi_c2(s) : 0;
+    const long long dx = Z[g.dim * (size_t)i] - Z[g.dim * (size_t)j], dy = Z[g.dim * (size_t)i + 1] - Z[g.dim * (size_t)j + 1];
+    const long long dz = g.dim == 3 ? Z[3 * (size_t)i + 2] - Z[3 * (size_t)j + 2] : 0;
+    if constexpr (FIXED == 1) {
+      const long long s = fx_dist2<3>(dx, dy, dz);
+      return s < FX_ONE_I ? fx_phi_c2(s) : 0;
+    } else {
+      const long long s = fx_dist2_wide<3>(dx, dy, dz);
+      return s < FX_EXP_END ? fx_exp_neg(s) : 0;
+    }
   } else {
     const int dim = g.dim;
     const double *xi = X + (size_t)i * dim, *xj = X + (size_t)j * dim;
@@ -847,7 +867,7 @@ __device__ __noinline__ int blk_diag(FxFactorShared &S, double *Fb, int J, int n
   return BlkCol<0>::run(S, q, Fb, J, nb, R, threadIdx.x & 31, *badrow, badrow);
 }
 /* Block column J minus the sums over the columns before it, for the rows i0 .. i0 + 63 (all warps). */
-template <bool FIXED>
+template <int FIXED>
 __device__ __noinline__ void blk_update(FxFactorShared &T, const lgb_geom &g, const unsigned *H, const double *X,
                                            long long *C, int m, int J, int i0)
 {
@@ -1016,7 +1036,8 @@ __global__ void __launch_bounds__(BLK_NT, 2) k_factor_blk(FactorParams P, int *n
       for (int j = tid; j < m; j += BLK_NT) {
         double cs = 0.0;
         for (int i = 0; i < m; i++)
-          cs += fabs((double)(P.fixed ? asm_entry<true>(g, X, i, j) : asm_entry<false>(g, X, i, j)));
+          cs += fabs((double)(P.fixed == 1 ? asm_entry<1>(g, X, i, j)
+                              : P.fixed == 2 ? asm_entry<2>(g, X, i, j) : asm_entry<0>(g, X, i, j)));
         cm = fmax(cm, cs * (1.0 / FX_ONE));
       }
       anorm = blk_reduce(cm, S.red, true);
@@ -1025,8 +1046,9 @@ __global__ void __launch_bounds__(BLK_NT, 2) k_factor_blk(FactorParams P, int *n
       const int nb = min(BLK_NB, m - J), rows = m - J, R = me - J, b = J / BLK_NB;
       double *Fb = Fq + fx_base(me, b);
       for (int i0 = J; i0 < m; i0 += BLK_ROWS) {
-        if (P.fixed) blk_update<true>(S.f, g, H, X, C, m, J, i0);
-        else blk_update<false>(S.f, g, H, X, C, m, J, i0);
+        if (P.fixed == 1) blk_update<1>(S.f, g, H, X, C, m, J, i0);
+        else if (P.fixed == 2) blk_update<2>(S.f, g, H, X, C, m, J, i0);
+        else blk_update<0>(S.f, g, H, X, C, m, J, i0);
       }
       __syncthreads();
       for (int q = tid; q < BLK_NB * BLK_NB; q += BLK_NT) {
@@ -1104,15 +1126,13 @@ extern "C" int lgb_op_factor(lgb_dev *d, void *stream)
   P.solved = d->solved;
   P.c64 = d->c64;
   P.c32 = d->c32;
+  P.cexp = d->cexp;
   P.fac = d->fac;
   P.ws = d->ws;
   P.ws_stride = d->ws_stride;
   P.ctrl = d->ctrl;
   P.kappa = d->cond_on ? d->kappa : NULL;
-  /* fixed-point coordinates eps (x - node) span |eps h|; 32 leaves the distances well inside 64 bits */
-  double ext = 0.0;
-  for (int i = 0; i < d->g.dim; i++) ext = fmax(ext, d->g.eps_r * d->g.h[i]);
-  P.fixed = d->g.kernel == LGB_KERNEL_WENDLAND_C2 && ext < 32.0;
+  P.fixed = d->fixed;
   /* one launch per patch-size class holding patches: its CTA size, grid and workspace slots */
   for (int c = 0; c < LGB_NCLS; c++) {
     if (d->cls_cap[c] <= 0 || d->cls_grid[c] <= 0) continue;

@@ -299,7 +299,7 @@ static void invalidate_graph(lgb_ctx *c)
 
 static void free_data(lgb_dev *d)
 {
-  DFREE(d->xd); DFREE(d->fd); DFREE(d->xs); DFREE(d->fs); DFREE(d->xr);
+  DFREE(d->xd); DFREE(d->fd); DFREE(d->xs); DFREE(d->fs); DFREE(d->xr); DFREE(d->xq);
   DFREE(d->cell_d); DFREE(d->sorted); DFREE(d->dtmp);
   d->nd_cap = 0;
 }
@@ -315,7 +315,8 @@ static void free_particles(lgb_dev *d)
 /* The dataset arrays a sharing context borrows (lagrbf_gpu_share_dataset). */
 static void borrow_dataset(lgb_dev *d, const lgb_dev *o)
 {
-  d->xd = o->xd; d->fd = o->fd; d->xs = o->xs; d->fs = o->fs; d->xr = o->xr;
+  d->xd = o->xd; d->fd = o->fd; d->xs = o->xs; d->fs = o->fs; d->xr = o->xr; d->xq = o->xq;
+  d->cexp = o->cexp;
   d->cell_d = o->cell_d; d->cstart = o->cstart; d->sorted = o->sorted;
   d->pm = o->pm; d->slot = o->slot; d->setup = o->setup; d->solved = o->solved;
   d->coff = o->coff; d->foff = o->foff; d->c64 = o->c64; d->c32 = o->c32; d->fac = o->fac;
@@ -329,6 +330,8 @@ static void unborrow_dataset(lgb_dev *d)
 {
   d->xd = d->fd = d->xs = d->fs = NULL;
   d->xr = NULL;
+  d->xq = NULL;
+  d->cexp = NULL;
   d->cell_d = d->cstart = d->sorted = NULL;
   d->pm = d->slot = d->setup = d->solved = NULL;
   d->coff = d->foff = NULL;
@@ -349,7 +352,7 @@ static void destroy_ctx(lgb_ctx *c)
   free_data(d);
   free_particles(d);
   DFREE(d->cstart); DFREE(d->dfill); DFREE(d->pm); DFREE(d->slot); DFREE(d->setup); DFREE(d->solved);
-  DFREE(d->need); DFREE(d->work); DFREE(d->work_s); DFREE(d->status); DFREE(d->coff); DFREE(d->foff); DFREE(d->c64); DFREE(d->kappa);
+  DFREE(d->need); DFREE(d->work); DFREE(d->work_s); DFREE(d->cexp); DFREE(d->status); DFREE(d->coff); DFREE(d->foff); DFREE(d->c64); DFREE(d->kappa);
   DFREE(d->c32); DFREE(d->fac); DFREE(d->ws); DFREE(d->pcount); DFREE(d->pstart); DFREE(d->pfill);
   DFREE(d->chunk_start); DFREE(d->scan_tmp); DFREE(d->scan_tmp64); DFREE(d->ctrl);
   DFREE(d->rec32); DFREE(d->rec_off); DFREE(d->bkey_buf); DFREE(d->cls_off_dev); DFREE(d->cdirty);
@@ -481,6 +484,10 @@ static int read_options(lgb_ctx *c)
   if (opt_int("solve_method", &k)) d->solve_method = k;
   if (d->solve_method < 0 || d->solve_method > 2) return set_error(LAGRBF_ERR_ARG_OUTOFRANGE, "unknown solve method %d", k);
   d->keep_factors = (d->solve_method != LGB_A_KSP_ASMB);
+  d->fixed = g->kernel == LGB_KERNEL_WENDLAND_C2 ? 1 : g->kernel == LGB_KERNEL_GAUSSIAN ? 2 : 0;
+  for (i = 0; i < dim; i++)
+    if (!(g->eps_r * g->h[i] < 32.0) || !(g->eps_w * g->h[i] < 32.0)) d->fixed = 0;
+  if (g->wr > 8) d->fixed = 0; /* the weights of the support nodes add up to less than 2^7 */
   d->F = 0;
   opt_int("n_interpolation_fields", &d->F);
   if (d->F < 0) return set_error(LAGRBF_ERR_ARG_OUTOFRANGE, "n_interpolation_fields must be >= 0");
@@ -568,6 +575,7 @@ static int create_ctx(lgb_ctx **out)
   d->need = (int *)dalloc(sizeof(int) * 2 * (size_t)nn, &err);
   d->work = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
   d->work_s = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
+  d->cexp = (int *)dalloc(sizeof(int) * (size_t)nn * (d->F > 0 ? d->F : 1), &err);
   d->status = (int *)dalloc(sizeof(int) * (size_t)nn, &err);
   d->coff = (long long *)dalloc(sizeof(long long) * (size_t)(nn + 1), &err);
   d->foff = (long long *)dalloc(sizeof(long long) * (size_t)(nn + 1), &err);
@@ -883,6 +891,7 @@ static int fill_data(lgb_ctx *c, int n, const double *coords, const double *valu
     d->xs = (double *)dalloc(sizeof(double) * (size_t)n * dim, &err);
     d->fs = (double *)dalloc(sizeof(double) * (size_t)n * (F ? F : 1), &err);
     d->xr = (float *)dalloc(sizeof(float) * 4 * (size_t)n, &err);
+    if (d->fixed) d->xq = (long long *)dalloc(sizeof(long long) * (size_t)n * dim, &err);
     d->cell_d = (int *)dalloc(sizeof(int) * (size_t)n, &err);
     d->sorted = (int *)dalloc(sizeof(int) * (size_t)n, &err);
     d->dtmp = (int *)dalloc(sizeof(int) * (size_t)n, &err);
@@ -928,39 +937,49 @@ static int fill_data(lgb_ctx *c, int n, const double *coords, const double *valu
   return 0;
 }
 
-/* Work-unit capacity of the evaluation kernel from the particles-per-cell histogram: the cost of a
-   capacity C = 64m (m = 1..4, R = 2 particles per thread) is, per work unit, one warp-equivalent of
-   block staging plus its active warps plus a third of a warp for each warp left without particles
-   (it still stages and occupies the SM). */
+/* Work-unit capacity of the evaluation kernel from the particles-per-cell histogram.
+   Fixed-point FP64 path (128 threads, warps without particles share the records of the others): the
+   largest of 128, 64 and 32 that gives every SM its four CTAs, so that small sets spread over the chip
+   (step over 10,000 particles in 49 cells: see lgb_evalfx.cuh).
+   Otherwise the cost of a capacity C = 64m (m = 1..4, R = 2 particles per thread) is, per work unit,
+   one warp-equivalent of block staging plus its active warps plus a third of a warp for each warp
+   left without particles (it still stages and occupies the SM). */
 static int choose_chunk(lgb_ctx *c)
 {
   lgb_dev *d = &c->d;
-  int nc = d->g.ncells, i, m, best = 4;
+  int nc = d->g.ncells, i, m, cap = 64 * 4;
   double bestcost = -1.0;
+  const int fx = d->prec != LGB_PREC_FP32 && d->fixed, most = fx ? 128 : LGB_CHUNK_MAX;
+  const char *env = getenv("LAGRBF_CHUNK");
   int *cnt = (int *)malloc(sizeof(int) * (size_t)(nc + 1));
   if (!cnt) return set_error(LAGRBF_ERR_MEM, "out of host memory");
   CUF(cudaMemcpyAsync(cnt, d->pstart, sizeof(int) * (size_t)(nc + 1), cudaMemcpyDeviceToHost, c->stream), free(cnt));
   CUF(cudaStreamSynchronize(c->stream), free(cnt));
-  for (m = 4; m >= 1; m--) {
-    double cost = 0.0;
-    int cap = 64 * m, twarps = 2 * m;
-    for (i = 0; i < nc; i++) {
-      int n = cnt[i + 1] - cnt[i], nch, per, aw;
-      if (n <= 0) continue;
-      nch = (n + cap - 1) / cap;
-      per = (n + nch - 1) / nch;
-      aw = ((per + 1) / 2 + 31) / 32;
-      cost += nch * (1.0 + aw + (twarps - aw) / 3.0);
+  if (fx) {
+    for (cap = 128; cap > 32; cap /= 2) {
+      long long units = 0;
+      for (i = 0; i < nc; i++) units += (cnt[i + 1] - cnt[i] + cap - 1) / cap;
+      if (units >= 4LL * d->nsm) break;
     }
-    if (bestcost < 0.0 || cost < bestcost * 0.98) { bestcost = cost; best = m; }
+  } else {
+    for (m = 4; m >= 1; m--) {
+      double cost = 0.0;
+      int twarps = 2 * m, cm = 64 * m;
+      for (i = 0; i < nc; i++) {
+        int n = cnt[i + 1] - cnt[i], nch, per, aw;
+        if (n <= 0) continue;
+        nch = (n + cm - 1) / cm;
+        per = (n + nch - 1) / nch;
+        aw = ((per + 1) / 2 + 31) / 32;
+        cost += nch * (1.0 + aw + (twarps - aw) / 3.0);
+      }
+      if (bestcost < 0.0 || cost < bestcost * 0.98) { bestcost = cost; cap = cm; }
+    }
   }
   free(cnt);
-  {
-    const char *env = getenv("LAGRBF_CHUNK");
-    if (env && atoi(env) >= 64 && atoi(env) <= LGB_CHUNK_MAX) best = atoi(env) / 64;
-  }
-  if (64 * best != d->chunk_cap) {
-    d->chunk_cap = 64 * best;
+  if (env && atoi(env) >= 64 && atoi(env) <= most) cap = atoi(env) / 64 * 64;
+  if (cap != d->chunk_cap) {
+    d->chunk_cap = cap;
     invalidate_graph(c);
     OP(lgb_op_bin_particles(d, 0, c->stream)); /* chunk offsets for the new capacity */
   }
@@ -1715,8 +1734,13 @@ LAGRBF_EXPORT int lagrbf_gpu_set_precision(void *ctx, int fp32)
   lgb_ctx *c = (lgb_ctx *)ctx;
   if (!c) return set_error(LAGRBF_ERR_ARG_NULL, "context is NULL");
   CU(cudaStreamSynchronize(c->stream));
+  if (c->d.prec == (fp32 ? LGB_PREC_FP32 : LGB_PREC_FP64)) return 0;
   c->d.prec = fp32 ? LGB_PREC_FP32 : LGB_PREC_FP64;
   invalidate_graph(c);
+  if (c->points_filled) {
+    TRY(choose_chunk(c)); /* the work-unit capacity depends on the precision */
+    CU(cudaStreamSynchronize(c->stream));
+  }
   return 0;
 }
 
@@ -1746,6 +1770,7 @@ LAGRBF_EXPORT int lagrbf_gpu_share_dataset(void *ctx, void *owner)
   free_data(d);
   DFREE(d->cstart); DFREE(d->pm); DFREE(d->slot); DFREE(d->setup); DFREE(d->solved);
   DFREE(d->coff); DFREE(d->foff); DFREE(d->c64); DFREE(d->c32); DFREE(d->fac); DFREE(d->rec32); DFREE(d->rec_off);
+  DFREE(d->cexp);
   borrow_dataset(d, &o->d);
   d->setup_all = 1; /* every patch of the borrowed dataset is set up: nothing is queued */
   c->shared_from = o;

@@ -66,6 +66,7 @@ static inline LGB_HD int lgb_patch_class(int m)
   while (c < LGB_NCLS - 1 && m > (32 << c)) c++;
   return c;
 }
+#define LGB_CEXP_NAN 0x7fffffff
 /* 8-byte elements of the blocked kernel's stored factor of m points (layout in lgb_factor.cu). */
 static inline LGB_HD long long lgb_fx_size(int m)
 {
@@ -156,6 +157,10 @@ typedef struct {
   float *xr;
   int *cell_d, *cstart, *sorted, *dfill, *dtmp;
   int max_cell_pts;
+  int fixed;           /* FP64 path in fixed point (lgb_fx.cuh): Wendland C2 or Gaussian kernel of
+                          moderate extent (eps_r h < 32: scaled coordinates of a block within +-64) */
+  long long *xq;       /* [nd*dim] eps_r (x - own cell's origin) in fixed point, cell order */
+  int *cexp;           /* [nnodes*F] |coefficients of the patch and field| < 2^cexp (or LGB_CEXP_NAN) */
   /* patches */
   int *pm, *slot, *setup, *solved, *work, *work_s, *status;
   int *need;          /* 2*nnodes ints: flags, also borrowed as nnodes int64 scratch */
