@@ -105,6 +105,32 @@ __host__ __device__ constexpr int vs_mask(int dim, int vs)
   return einv_mask(dim, vs_off(dim, vs)) & ((dim == 3 && vs == 13) ? 0x0F : (dim == 3 && vs == 14) ? 0xF0 : 0xFF);
 }
 template <int DIM> struct VGeo { static constexpr int NVS = LGB_NVSEG(DIM); };
+/* The masks of the virtual segments and of the neighbour offsets as tables: evaluated at run time the
+   expressions above cost hundreds of instructions. */
+struct EMasks {
+  unsigned char vs[2][28], off[2][27];
+  constexpr EMasks() : vs(), off()
+  {
+    for (int dim = 2; dim <= 3; dim++) {
+      for (int v = 0; v < LGB_NVSEG(dim); v++) vs[dim - 2][v] = (unsigned char)vs_mask(dim, v);
+      for (int o = 0; o < (dim == 3 ? 27 : 9); o++) off[dim - 2][o] = (unsigned char)einv_mask(dim, o);
+    }
+  }
+};
+static __constant__ EMasks c_masks;
+
+/* Sum over the neighbour offsets of points x set-up corner patches (one warp; the algorithmic count of
+   coefficient products per field and particle). */
+template <int DIM>
+__device__ __forceinline__ long long emask_products(const int *cnt, const int *setup)
+{
+  const int lane = threadIdx.x & 31;
+  const unsigned on = __ballot_sync(0xffffffffu, lane < EGeo<DIM>::NEN && setup[lane & 7]);
+  long long v = lane < EGeo<DIM>::NOFF ? (long long)cnt[lane] * __popc(c_masks.off[DIM - 2][lane] & on) : 0;
+  for (int w = 16; w > 0; w >>= 1) v += __shfl_xor_sync(0xffffffffu, v, w);
+  return v;
+}
+
 /* Record length (elements) for a neighbour offset: 4 coordinates + ninv*FP coefficients, padded
    to a 16-byte multiple. */
 template <typename Real> __host__ __device__ constexpr int erec(int ninv, int fp)

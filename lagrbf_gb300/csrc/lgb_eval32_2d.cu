@@ -27,30 +27,31 @@ static int launch32(const EvalParams &P, int grid, cudaStream_t s)
   return launch32r<DIM, FP, KER, 2>(P, grid, s);
 }
 
-/* The record-streamed kernel: EVR_NB stages of P.budget floats, then the PU-weight pairs. */
-template <int DIM, int KER>
+/* The record-streamed kernel: EVR_NB stages of P.budget floats, the PU weights and the shares' support
+   sums (10 words per thread). */
+template <int DIM, int KER, int RM>
 static int launch_rec(const EvalParams &P, int grid, cudaStream_t s)
 {
   /* the attribute is set once to the device's largest opt-in size (threads racing on it all set the
      same value; a per-call size could shrink it under another thread's launch) */
   static int attr = 0;
-  const size_t smem = (size_t)EVR_NB * P.budget * sizeof(float) + (size_t)(P.chunk_cap / 2) * ((1 << DIM) + 1) * 8;
+  const size_t smem = ((size_t)EVR_NB * P.budget + (size_t)P.chunk_cap * 10) * sizeof(float);
   if (!attr) {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncSetAttribute(k_eval_rec<DIM, DIM, KER>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaFuncSetAttribute(k_eval_rec<DIM, DIM, KER, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          optin - 8192);
     attr = 1;
   }
-  k_eval_rec<DIM, DIM, KER><<<grid, P.chunk_cap / 2, smem, s>>>(P);
+  k_eval_rec<DIM, DIM, KER, RM><<<grid, P.chunk_cap / RM, smem, s>>>(P);
   return (int)cudaGetLastError();
 }
 
 template <int DIM, int KER>
 static int launch32_fp(const EvalParams &P, int fp, int stage, int grid, cudaStream_t s)
 {
-  if (stage == 1) return launch_rec<DIM, KER>(P, grid, s); /* records hold the dim velocity fields */
+  if (stage == 1) return P.chunk_cap <= 128 ? launch_rec<DIM, KER, 1>(P, grid, s) : launch_rec<DIM, KER, 2>(P, grid, s); /* records hold the dim velocity fields */
   switch (fp) {
   case 1: return launch32<DIM, 1, KER>(P, grid, s);
   case 2: return launch32<DIM, 2, KER>(P, grid, s);

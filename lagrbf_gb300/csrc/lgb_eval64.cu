@@ -53,7 +53,7 @@ static int tma_budget(void)
   static int b = -1;
   if (b < 0) {
     const char *e = getenv("LAGRBF_TMA_BUDGET");
-    b = (e && atoi(e) >= 256) ? (atoi(e) / 4) * 4 : BUDGET32_TMA;
+    b = (e && atoi(e) >= 1024) ? (atoi(e) / 4) * 4 : BUDGET32_TMA;
   }
   return b;
 }
@@ -99,7 +99,7 @@ extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int ou
     int rc;
     if (d->prec == LGB_PREC_FP32) {
       const int stage = (d->rec32 && f == 0 && fp == g.dim && d->rec_fp == g.dim) ? 1 : 0;
-      P.budget = stage ? tma_budget() : BUDGET32;
+      P.budget = stage ? tma_budget() * d->chunk_cap / 128 : BUDGET32; /* the ring grows with the unit */
       rc = (g.dim == 3) ? lgb_eval32_launch_3d(&P, fp, ker, stage, grid, stream)
                         : lgb_eval32_launch_2d(&P, fp, ker, stage, grid, stream);
     } else if (d->fixed) {

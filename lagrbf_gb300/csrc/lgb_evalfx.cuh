@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
       while (vs < NVS) {
         const int c = S.cnt[vs_off(DIM, vs)] - pp;
         if (c <= 0) { vs++; pp = 0; continue; }
-        const int len = fxe_len(DIM, __popc(vs_mask(DIM, vs)), FP), fit = (FXE_BUDGET - base) / len;
+        const int len = fxe_len(DIM, __popc(c_masks.vs[DIM - 2][vs]), FP), fit = (FXE_BUDGET - base) / len;
         if (fit <= 0) break;
         const int take = min(c, fit);
         S.seg_v[nseg] = vs; S.seg_p0[nseg] = pp; S.seg_n[nseg] = take; S.seg_base[nseg] = base;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     const int nseg = S.nseg;
     if (nseg == 0) break;
     for (int i = 0; i < nseg; i++) {
-      const int vs = S.seg_v[i], o = vs_off(DIM, vs), mask = vs_mask(DIM, vs), ni = __popc(mask);
+      const int vs = S.seg_v[i], o = vs_off(DIM, vs), mask = c_masks.vs[DIM - 2][vs], ni = __popc(mask);
       const int len = fxe_len(DIM, ni, FP), n = S.seg_n[i], p0 = S.seg_p0[i];
       unsigned char *dst = smem_raw + S.seg_base[i];
       for (int t = tid; t < n * DIM; t += FXE_T) {
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     __syncthreads();
     if (active)
       for (int i = 0; i < nseg; i++) {
-        const int mask = vs_mask(DIM, S.seg_v[i]), n = S.seg_n[i];
+        const int mask = c_masks.vs[DIM - 2][S.seg_v[i]], n = S.seg_n[i];
         const unsigned char *rec = smem_raw + S.seg_base[i];
         const double *w = &S.w[0][idx];
         switch (__popc(mask)) {
@@ -299,14 +299,9 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
   for (int off = 16; off > 0; off >>= 1) wloc += __shfl_down_sync(0xffffffffu, wloc, off);
   if (lane == 0) atomicAdd(&S.wsum, wloc);
   __syncthreads();
-  if (tid == 0) {
-    long long msum = 0;
-    for (int o = 0; o < NOFF; o++) {
-      const int mask = einv_mask(DIM, o);
-      int ninv = 0;
-      for (int k = 0; k < NEN; k++) ninv += ((mask >> k) & 1) && S.setup[k];
-      msum += (long long)S.cnt[o] * ninv;
-    }
+  if (tid < 32) {
+    const long long msum = emask_products<DIM>(S.cnt, S.setup);
+    if (tid > 0) return;
     const double kphi = KER == KER_GAUSS ? 4.0 : 8.0;
     const double fl = (double)pn * ((double)S.blk * (10.0 + kphi) + 2.0 * FP * (double)msum + NEN * (2.0 * FP + 1.0)) +
                       18.0 * (double)S.wsum;

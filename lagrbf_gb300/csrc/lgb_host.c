@@ -834,7 +834,7 @@ static int ensure_records(lgb_ctx *c)
       ninv = (a == 0 ? 2 : 1) * (b == 0 ? 2 : 1) * ((g->dim == 3 && e == 0) ? 2 : 1);
       if (ninv > 4) ninv = 4;
       S = LGB_REC2_LEN(g->dim, ninv, g->dim);
-      total += (long long)(cs[nb + 1] - cs[nb]) * S;
+      total += (long long)((cs[nb + 1] - cs[nb] + 1) / 2) * S;
     }
   }
   off[nc] = total;
@@ -938,31 +938,59 @@ static int fill_data(lgb_ctx *c, int n, const double *coords, const double *valu
 }
 
 /* Work-unit capacity of the evaluation kernel from the particles-per-cell histogram.
-   Fixed-point FP64 path (128 threads, warps without particles share the records of the others): the
-   largest of 128, 64 and 32 that gives every SM its four CTAs, so that small sets spread over the chip
-   (step over 10,000 particles in 49 cells: see lgb_evalfx.cuh).
-   Otherwise the cost of a capacity C = 64m (m = 1..4, R = 2 particles per thread) is, per work unit,
-   one warp-equivalent of block staging plus its active warps plus a third of a warp for each warp
-   left without particles (it still stages and occupies the SM). */
+   Fixed-point FP64 kernel (128 threads, threads without particles share the records of the others):
+   the largest of 128, 64 and 32 that gives every SM its four CTAs, so that small sets spread over the
+   chip.
+   FP32 record kernel (as many threads as the capacity up to 128, shared in the same way; 256: two
+   particles per thread): 128 threads for sets of so few units that the shares shorten the launch,
+   else the smallest of 32, 64 and 128 that holds a mean cell, so that units of sparse cells cost no
+   idle warps (1M particles of a mixture over 970,000 cells: 32 threads 4.0 ms per launch, 128 threads
+   23.5 ms).  From 128 particles per cell on, 128 or 256 by the warps their units keep busy, where
+   two particles per thread cost 1.8 of one (563 per cell, 16.8M particles: 256 22.6 ms, 128 25.1 ms;
+   144 per cell, 2M particles: 128 3.4 ms, 256 4.7 ms).
+   Gather kernels: the cost of a capacity C = 64m (m = 1, 2) is, per work unit, one warp-equivalent of
+   block staging plus its active warps plus a third of a warp for each warp left without particles
+   (it still stages and occupies the SM). */
+static double unit_warps(int n); /* warps that a unit of n <= 128 particles keeps busy */
 static int choose_chunk(lgb_ctx *c)
 {
   lgb_dev *d = &c->d;
-  int nc = d->g.ncells, i, m, cap = 64 * 4;
+  int nc = d->g.ncells, i, m, cap = LGB_CHUNK_MAX;
   double bestcost = -1.0;
-  const int fx = d->prec != LGB_PREC_FP32 && d->fixed, most = fx ? 128 : LGB_CHUNK_MAX;
+  const int fx = d->prec == LGB_PREC_FP32 ? d->F >= d->g.dim : d->fixed;
   const char *env = getenv("LAGRBF_CHUNK");
   int *cnt = (int *)malloc(sizeof(int) * (size_t)(nc + 1));
   if (!cnt) return set_error(LAGRBF_ERR_MEM, "out of host memory");
   CUF(cudaMemcpyAsync(cnt, d->pstart, sizeof(int) * (size_t)(nc + 1), cudaMemcpyDeviceToHost, c->stream), free(cnt));
   CUF(cudaStreamSynchronize(c->stream), free(cnt));
-  if (fx) {
+  if (fx && d->prec == LGB_PREC_FP32) {
+    long long units = 0, used = 0, n = 0;
+    for (i = 0; i < nc; i++) {
+      units += (cnt[i + 1] - cnt[i] + 127) / 128;
+      used += cnt[i + 1] > cnt[i];
+      n += cnt[i + 1] - cnt[i];
+    }
+    cap = 128;
+    if (units >= 4LL * d->nsm)
+      for (cap = 32; cap < LGB_CHUNK_MAX && n > cap * used; cap *= 2) ;
+    if (cap > 128) {
+      double c1 = 0.0, c2 = 0.0;
+      for (i = 0; i < nc; i++) {
+        n = cnt[i + 1] - cnt[i];
+        c1 += 4.0 * (double)(n / 128) + unit_warps((int)(n % 128));
+        c2 += 7.2 * (double)(n / 256) + (n % 256 > 128 ? 7.2 : unit_warps((int)(n % 256)));
+      }
+      if (c1 <= c2) cap = 128;
+    }
+    if (!d->rec32 && cap < 64) cap = 64; /* gather kernel */
+  } else if (fx) {
     for (cap = 128; cap > 32; cap /= 2) {
       long long units = 0;
       for (i = 0; i < nc; i++) units += (cnt[i + 1] - cnt[i] + cap - 1) / cap;
       if (units >= 4LL * d->nsm) break;
     }
   } else {
-    for (m = 4; m >= 1; m--) {
+    for (m = LGB_CHUNK_MAX / 64; m >= 1; m--) {
       double cost = 0.0;
       int twarps = 2 * m, cm = 64 * m;
       for (i = 0; i < nc; i++) {
@@ -977,7 +1005,7 @@ static int choose_chunk(lgb_ctx *c)
     }
   }
   free(cnt);
-  if (env && atoi(env) >= 64 && atoi(env) <= most) cap = atoi(env) / 64 * 64;
+  if (env && (atoi(env) == 64 || atoi(env) == 128 || (atoi(env) == 256 && !(fx && d->prec != LGB_PREC_FP32)))) cap = atoi(env);
   if (cap != d->chunk_cap) {
     d->chunk_cap = cap;
     invalidate_graph(c);
@@ -985,6 +1013,15 @@ static int choose_chunk(lgb_ctx *c)
   }
   d->max_chunks = d->g.ncells + (d->np + d->chunk_cap - 1) / d->chunk_cap + 1;
   return 0;
+}
+
+/* Up to 64 particles the shares divide the records, so a unit costs as its next power of two. */
+static double unit_warps(int n)
+{
+  int p2 = 1;
+  if (n > 64) return (double)((n + 31) / 32);
+  while (p2 < n) p2 *= 2;
+  return n > 0 ? p2 / 32.0 : 0.0;
 }
 
 static int fill_points(lgb_ctx *c, int n, const double *coords, const double *values, const int64_t *pidx)

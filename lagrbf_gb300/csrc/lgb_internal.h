@@ -40,8 +40,8 @@ enum { LGB_VF_NONE = 0, LGB_VF_ROTATION = 1, LGB_VF_CELLULAR = 2, LGB_VF_ABC = 3
 
 /* FP32 record blocks streamed by the evaluation kernel (lgb_evalrec.cuh): per cell, the data
    points of its 3^dim neighbour cells in LGB_NVSEG virtual segments (3D: the centre cell twice,
-   with the coefficients of corners 0-3 and of corners 4-7); a record is 2*dim coordinate floats
-   and 2 floats per (field, involved patch), padded to 16 bytes. */
+   with the coefficients of corners 0-3 and of corners 4-7); a record holds two points: 2*dim
+   coordinate floats and 2 floats per (field, involved patch), padded to 16 bytes. */
 #define LGB_NVSEG(dim) ((dim) == 3 ? 28 : 9)
 #define LGB_REC2_LEN(dim, ninv, fp) (((2 * (dim) + 2 * (ninv) * (fp) + 3) / 4) * 4)
 /* Patch-size classes of the set-up / solve launches: class c holds the patches of up to
