@@ -55,6 +55,7 @@ struct EvalParams {
   lgb_ctrl *ctrl;
   int budget;             /* staging budget, elements of the compute type (per buffer) */
   int chunk_cap;          /* particles per work unit (blockDim.x * R)     */
+  int threads;            /* of a work unit of the record kernel */
   float *rec32;           /* precomputed FP32 record blocks (streamed by k_eval_rec) */
   const long long *rec_off;
   int poll_limit;         /* polls of a bounded mbarrier wait before it gives up          */
@@ -97,23 +98,29 @@ __host__ __device__ constexpr int eslot(int dim, int k, int o)
   return (eoff_a(o) - ecorner_ox(k) + 1) + 2 * (eoff_b(o) - ecorner_oy(k) + 1) +
          (dim == 3 ? 4 * (eoff_e(dim, o) - ecorner_oz(dim, k) + 1) : 0);
 }
-/* Virtual segments: the neighbour offsets, in 3D with the centre cell (in all eight corner patches)
-   twice, for corners 0-3 and 4-7, so that a segment involves at most four patches. */
-__host__ __device__ constexpr int vs_off(int dim, int vs) { return (dim == 3 && vs > 13) ? vs - 1 : vs; }
-__host__ __device__ constexpr int vs_mask(int dim, int vs)
-{
-  return einv_mask(dim, vs_off(dim, vs)) & ((dim == 3 && vs == 13) ? 0x0F : (dim == 3 && vs == 14) ? 0xF0 : 0xFF);
-}
+/* Virtual segments: the neighbour offsets by the number of patches that they are in (cells that share a
+   vertex, an edge, a face with the evaluating cell, that cell), so that the segments that threads of a warp
+   work on side by side have records of one length.  In 3D the centre cell (in all eight corner patches) is
+   there twice, for corners 0-3 and 4-7: a segment involves at most four patches. */
 template <int DIM> struct VGeo { static constexpr int NVS = LGB_NVSEG(DIM); };
-/* The masks of the virtual segments and of the neighbour offsets as tables: evaluated at run time the
-   expressions above cost hundreds of instructions. */
+/* Neighbour offset and mask of the virtual segments, and the masks of the neighbour offsets, as tables:
+   evaluated at run time the expressions cost hundreds of instructions. */
 struct EMasks {
-  unsigned char vs[2][28], off[2][27];
-  constexpr EMasks() : vs(), off()
+  unsigned char vo[2][28], vs[2][28], off[2][27];
+  constexpr EMasks() : vo(), vs(), off()
   {
     for (int dim = 2; dim <= 3; dim++) {
-      for (int v = 0; v < LGB_NVSEG(dim); v++) vs[dim - 2][v] = (unsigned char)vs_mask(dim, v);
-      for (int o = 0; o < (dim == 3 ? 27 : 9); o++) off[dim - 2][o] = (unsigned char)einv_mask(dim, o);
+      const int no = dim == 3 ? 27 : 9;
+      int v = 0;
+      for (int o = 0; o < no; o++) off[dim - 2][o] = (unsigned char)einv_mask(dim, o);
+      for (int ni = 1; ni <= 8; ni *= 2)
+        for (int o = 0; o < no; o++) {
+          if (epopc(einv_mask(dim, o)) != ni) continue;
+          for (int half = 0; half < (ni == 8 ? 2 : 1); half++, v++) {
+            vo[dim - 2][v] = (unsigned char)o;
+            vs[dim - 2][v] = (unsigned char)(einv_mask(dim, o) & (ni < 8 ? 0xFF : half ? 0xF0 : 0x0F));
+          }
+        }
     }
   }
 };

@@ -35,7 +35,7 @@ static int launch_rec(const EvalParams &P, int grid, cudaStream_t s)
   /* the attribute is set once to the device's largest opt-in size (threads racing on it all set the
      same value; a per-call size could shrink it under another thread's launch) */
   static int attr = 0;
-  const size_t smem = ((size_t)EVR_NB * P.budget + (size_t)P.chunk_cap * 10) * sizeof(float);
+  const size_t smem = ((size_t)EVR_NB * P.budget + (size_t)(RM == 2 ? 2 * EVR_T : P.threads) * 10) * sizeof(float);
   if (!attr) {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
@@ -44,14 +44,17 @@ static int launch_rec(const EvalParams &P, int grid, cudaStream_t s)
                          optin - 8192);
     attr = 1;
   }
-  k_eval_rec<DIM, DIM, KER, RM><<<grid, P.chunk_cap / RM, smem, s>>>(P);
+  k_eval_rec<DIM, DIM, KER, RM><<<grid, P.threads, smem, s>>>(P);
   return (int)cudaGetLastError();
 }
 
 template <int DIM, int KER>
 static int launch32_fp(const EvalParams &P, int fp, int stage, int grid, cudaStream_t s)
 {
-  if (stage == 1) return P.chunk_cap <= 128 ? launch_rec<DIM, KER, 1>(P, grid, s) : launch_rec<DIM, KER, 2>(P, grid, s); /* records hold the dim velocity fields */
+  if (stage == 1) { /* records hold the dim velocity fields */
+    if (P.threads > EVR_T) return launch_rec<DIM, KER, 0>(P, grid, s);
+    return P.chunk_cap <= EVR_T ? launch_rec<DIM, KER, 1>(P, grid, s) : launch_rec<DIM, KER, 2>(P, grid, s);
+  }
   switch (fp) {
   case 1: return launch32<DIM, 1, KER>(P, grid, s);
   case 2: return launch32<DIM, 2, KER>(P, grid, s);

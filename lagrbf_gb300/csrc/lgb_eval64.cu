@@ -90,6 +90,7 @@ extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int ou
     P.out_stride = out_stride;
     P.ctrl = d->ctrl;
     P.chunk_cap = d->chunk_cap;
+    P.threads = d->unit_threads;
     P.rec32 = d->rec32;
     P.rec_off = d->rec_off;
     P.poll_limit = d->eval_poll_limit > 0 ? d->eval_poll_limit : EVAL_POLL_LIMIT;
@@ -99,7 +100,8 @@ extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int ou
     int rc;
     if (d->prec == LGB_PREC_FP32) {
       const int stage = (d->rec32 && f == 0 && fp == g.dim && d->rec_fp == g.dim) ? 1 : 0;
-      P.budget = stage ? tma_budget() * d->chunk_cap / 128 : BUDGET32; /* the ring grows with the unit */
+      /* the ring grows with the unit, and for more than 128 threads so that their streams find segments in it */
+      P.budget = !stage ? BUDGET32 : d->unit_threads > 128 ? d->unit_threads * 32 : tma_budget() * d->chunk_cap / 128;
       rc = (g.dim == 3) ? lgb_eval32_launch_3d(&P, fp, ker, stage, grid, stream)
                         : lgb_eval32_launch_2d(&P, fp, ker, stage, grid, stream);
     } else if (d->fixed) {

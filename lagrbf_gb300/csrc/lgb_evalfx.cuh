@@ -15,18 +15,19 @@
  * in shared memory: coordinates in units of the support radius relative to the evaluating cell's
  * origin, coefficients relative to a power of two above the largest one of the field in the cell's
  * patches, both fixed point, the coefficients as {hi, lo}.  Every lane reads the same record
- * (broadcast).  A segment's per-patch sums are exact 64-bit sums; after at most FXE_RUN records they
- * are folded into the particle's FP64 field sums with the PU weights.  Units with fewer particles than
- * lanes give every warp a share of the records (a cell of 20 particles would otherwise leave three of
- * four warps idle), and the shares are added at the end.  The PU weights are fixed point too: an exact
- * sum over the support nodes, which the shares divide among themselves.
+ * (broadcast).  A segment's per-patch sums are exact 64-bit sums; after FXE_RUN records they
+ * are folded, still as whole numbers, into the particle's field sums with the PU weights.  Units of up to 64
+ * particles divide the runs of records among their warps (a cell of 20 particles would otherwise leave three of
+ * four warps idle); whole numbers make the result independent of it, and so of the unit's other particles.
+ * The PU weights are fixed point too, divided at the end by an exact sum over the support nodes, which the
+ * shares divide among themselves.
  */
 #pragma once
 #include "lgb_eval.cuh"
 #include "lgb_fx.cuh"
 
 #define FXE_T 128       /* threads */
-#define FXE_RUN 120     /* records between folds: 120 products below 2^56 stay within 63 bits */
+#define FXE_RUN 32      /* records between folds (32 products below 2^56 stay within 63 bits) */
 #define FXE_BUDGET 24576 /* bytes of staged records */
 
 /* Bytes of a record: coordinates (3D: padded to 32), coefficients. */
@@ -41,9 +42,9 @@ struct FxeShared {
   int seg_v[28], seg_p0[28], seg_n[28], seg_base[28], nseg;
   int vs, pp;                /* planner cursor */
   int cell, pbeg, pn, blk, wsum;
-  double scale[4];           /* 2^(exps - 56), NaN where a coefficient is not finite */
+  double scale[4];           /* units of the field sums, NaN where a coefficient is not finite */
   unsigned long long den[FXE_T];
-  double w[8][FXE_T];        /* PU weights */
+  unsigned long long w[8][FXE_T]; /* phiW of the corners */
 };
 
 template <int DIM, int KER>
@@ -58,20 +59,35 @@ __device__ __forceinline__ long long fxe_phi(long long dx, long long dy, long lo
   }
 }
 
-/* n records of NI patches at rec for the lane's particle, from share sh of ns on; the per-patch sums
-   are folded into val with the PU weights w[corner * FXE_T]. */
+/* S w / 2^(64 - FXE_FINE), rounded, for a sum |S| < 2^61 and a weight w < 2^63.  The Gaussian kernel's sums cancel more:
+   three bits finer (relative error of a field against long double, 2D, 350 points per patch: 2.6e-16; FP64
+   3.2e-16; without them 3.9e-16; Wendland C2 2.2e-13 without, FP64 6.0e-13). */
+template <int KER> constexpr int fxe_fine = KER == KER_GAUSS ? 3 : 0;
+template <int KER>
+__device__ __forceinline__ long long fxe_weigh(long long s, unsigned long long w)
+{
+  constexpr int F = fxe_fine<KER>;
+  const long long hi = (long long)__umul64hi((unsigned long long)s, w) - (s < 0 ? (long long)w : 0ll);
+  return (hi << F) + (long long)(((((unsigned long long)s * w) >> (63 - F)) + 1) >> 1);
+}
+
+/* The runs of FXE_RUN records of a piece (n records of NI patches at rec) whose number is the share's (run: of
+   the round, so far), for the lane's particle: the per-patch sums of a run are folded into val, two words per
+   field, with the PU weights w[corner * FXE_T].  A run's fold is a whole number that does not depend on which
+   share does it, and so neither does their sum. */
 template <int DIM, int FP, int KER, int NI>
-__device__ __forceinline__ void fxe_segment(const unsigned char *rec, int n, int sh, int ns, long long px, long long py,
-                                            long long pz, unsigned mask, const double *w, double (&val)[FP])
+__device__ __forceinline__ void fxe_segment(const unsigned char *rec, int n, int sh, int ns, int &run, long long px, long long py,
+                                            long long pz, unsigned mask, const unsigned long long *w, int ws, long long (&val)[FP][2])
 {
   constexpr int LEN = fxe_len(DIM, NI, FP), HEAD = DIM == 3 ? 32 : 16;
-  for (int p0 = sh; p0 < n; p0 += ns * FXE_RUN) {
-    const int p1 = min(n, p0 + ns * FXE_RUN);
+  for (int p0 = 0; p0 < n; p0 += FXE_RUN, run++) {
+    if ((run & (ns - 1)) != sh) continue;
+    const int p1 = min(n, p0 + FXE_RUN);
     long long hh[NI * FP], hl[NI * FP];
 #pragma unroll
     for (int q = 0; q < NI * FP; q++) { hh[q] = 0; hl[q] = 0; }
 #pragma unroll 1
-    for (int p = p0; p < p1; p += ns) {
+    for (int p = p0; p < p1; p++) {
       const unsigned char *r = rec + (size_t)p * LEN;
       const longlong2 xy = *reinterpret_cast<const longlong2 *>(r);
       const long long z = (DIM == 3) ? *reinterpret_cast<const long long *>(r + 16) : 0;
@@ -94,10 +110,14 @@ __device__ __forceinline__ void fxe_segment(const unsigned char *rec, int n, int
     unsigned m = mask;
 #pragma unroll
     for (int j = 0; j < NI; j++) {
-      const double wk = w[(__ffs(m) - 1) * FXE_T];
+      const unsigned long long wk = w[(__ffs(m) - 1) * FXE_T] << ws;
       m &= m - 1;
 #pragma unroll
-      for (int f = 0; f < FP; f++) val[f] = fma(wk, (double)fx_sum(hh[j * FP + f], hl[j * FP + f]), val[f]);
+      for (int f = 0; f < FP; f++) {
+        const long long v = fxe_weigh<KER>(fx_sum(hh[j * FP + f], hl[j * FP + f]), wk);
+        val[f][0] += v & 0xffffffffll;
+        val[f][1] += v >> 32;
+      }
     }
   }
 }
@@ -157,7 +177,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     for (int k = 0; k < NEN; k++)
       if (S.setup[k]) e = max(e, P.cexp[(size_t)S.node[k] * P.F + P.f0 + tid]);
     S.exps[tid] = e;
-    S.scale[tid] = e < 2000 ? __hiloint2double((1023 - 56 + e) << 20, 0) : __hiloint2double(0x7ff80000, 0);
+    S.scale[tid] = e < 2000 ? __hiloint2double((1023 + 8 - fxe_fine<KER> + e) << 20, 0) : __hiloint2double(0x7ff80000, 0);
   }
   if (tid == 32) {
     int nb = 0;
@@ -165,7 +185,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     S.blk = nb;
   }
   /* groups of 32 particles; a group's warps share its records and support nodes */
-  const int ng = (pn + 31) / 32, ns = FXE_T / 32 / ng, grp = warp % ng, sh = warp / ng;
+  const int ng = (pn + 31) / 32, ns = ng == 1 ? 4 : ng == 2 ? 2 : 1, grp = warp % ng, sh = warp / ng;
   const bool active = sh < ns;
   const int idx = 32 * grp + lane; /* lanes beyond the unit repeat its last particle */
   const int pid = P.plist[S.pbeg + min(idx, pn - 1)];
@@ -178,7 +198,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
   }
   S.den[tid] = 0ull;
 #pragma unroll
-  for (int k = 0; k < NEN; k++) S.w[k][tid] = 0.0; /* corners beyond the support */
+  for (int k = 0; k < NEN; k++) S.w[k][tid] = 0ull; /* corners beyond the support */
   __syncthreads();
   if (S.blk == 0) return; /* empty neighbourhood: the value is left untouched (interpolation.c:89) */
 
@@ -205,25 +225,26 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
       wloc += v > 0;
       const int a = ijk[0] - ci, b = ijk[1] - cj, e = ijk[2] - cl;
       if ((unsigned)a < 2 && (unsigned)b < 2 && (unsigned)e < 2)
-        S.w[(b ? 3 - a : a) + (DIM == 3 ? 4 * e : 0)][idx] = (double)v; /* corner of the cell */
+        S.w[(b ? 3 - a : a) + (DIM == 3 ? 4 * e : 0)][idx] = (unsigned long long)v; /* corner of the cell */
     }
     atomicAdd(&S.den[idx], den);
     if (idx >= pn) wloc = 0;
   }
   __syncthreads();
-  if (active) {
-    const double den = (double)(long long)S.den[idx];
-    for (int k = sh; k < NEN; k += ns) S.w[k][idx] = den > 0.0 ? S.w[k][idx] / den : 0.0;
-  }
-
-  double val[FP];
+  /* the support sum in bit 62; the division by it comes last */
+  unsigned long long wmax = 1;
 #pragma unroll
-  for (int f = 0; f < FP; f++) val[f] = 0.0;
+  for (int k = 0; k < NEN; k++) wmax = max(wmax, S.w[k][idx]);
+  const int ws = __clzll((long long)max(S.den[idx], wmax)) - 1;
+
+  long long val[FP][2];
+#pragma unroll
+  for (int f = 0; f < FP; f++) val[f][0] = val[f][1] = 0;
   for (;;) {
     if (tid == 0) { /* the next round of records */
       int vs = S.vs, pp = S.pp, base = 0, nseg = 0;
       while (vs < NVS) {
-        const int c = S.cnt[vs_off(DIM, vs)] - pp;
+        const int c = S.cnt[c_masks.vo[DIM - 2][vs]] - pp;
         if (c <= 0) { vs++; pp = 0; continue; }
         const int len = fxe_len(DIM, __popc(c_masks.vs[DIM - 2][vs]), FP), fit = (FXE_BUDGET - base) / len;
         if (fit <= 0) break;
@@ -241,7 +262,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     const int nseg = S.nseg;
     if (nseg == 0) break;
     for (int i = 0; i < nseg; i++) {
-      const int vs = S.seg_v[i], o = vs_off(DIM, vs), mask = c_masks.vs[DIM - 2][vs], ni = __popc(mask);
+      const int vs = S.seg_v[i], o = c_masks.vo[DIM - 2][vs], mask = c_masks.vs[DIM - 2][vs], ni = __popc(mask);
       const int len = fxe_len(DIM, ni, FP), n = S.seg_n[i], p0 = S.seg_p0[i];
       unsigned char *dst = smem_raw + S.seg_base[i];
       for (int t = tid; t < n * DIM; t += FXE_T) {
@@ -267,32 +288,37 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
       }
     }
     __syncthreads();
+    int run = 0;
     if (active)
       for (int i = 0; i < nseg; i++) {
         const int mask = c_masks.vs[DIM - 2][S.seg_v[i]], n = S.seg_n[i];
         const unsigned char *rec = smem_raw + S.seg_base[i];
-        const double *w = &S.w[0][idx];
+        const unsigned long long *w = &S.w[0][idx];
         switch (__popc(mask)) {
-        case 1: fxe_segment<DIM, FP, KER, 1>(rec, n, sh, ns, pq[0], pq[1], pq[2], mask, w, val); break;
-        case 2: fxe_segment<DIM, FP, KER, 2>(rec, n, sh, ns, pq[0], pq[1], pq[2], mask, w, val); break;
-        default: fxe_segment<DIM, FP, KER, 4>(rec, n, sh, ns, pq[0], pq[1], pq[2], mask, w, val); break;
+        case 1: fxe_segment<DIM, FP, KER, 1>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, ws, val); break;
+        case 2: fxe_segment<DIM, FP, KER, 2>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, ws, val); break;
+        default: fxe_segment<DIM, FP, KER, 4>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, ws, val); break;
         }
       }
     __syncthreads();
   }
 
-  /* the shares' sums (in share order) through the drained staging buffer */
-  double *red = reinterpret_cast<double *>(smem_raw);
+  /* the shares' sums through the drained staging buffer */
+  long long *red = reinterpret_cast<long long *>(smem_raw);
   if (active && sh > 0)
 #pragma unroll
-    for (int f = 0; f < FP; f++) red[((sh - 1) * FP + f) * FXE_T + idx] = val[f];
+    for (int f = 0; f < FP; f++)
+      for (int h = 0; h < 2; h++) red[(((sh - 1) * FP + f) * 2 + h) * (FXE_T / 2) + idx] = val[f][h];
   __syncthreads();
   if (active && sh == 0 && idx < pn) {
     double *o = P.out + (size_t)pid * P.out_stride;
+    const double den = (double)(long long)S.den[idx], sc = den > 0.0 ? __hiloint2double((1023 - ws) << 20, 0) / den : 0.0;
 #pragma unroll
     for (int f = 0; f < FP; f++) {
-      for (int k = 1; k < ns; k++) val[f] += red[((k - 1) * FP + f) * FXE_T + idx];
-      o[f] = val[f] * S.scale[f];
+      for (int k = 1; k < ns; k++)
+        for (int h = 0; h < 2; h++) val[f][h] += red[(((k - 1) * FP + f) * 2 + h) * (FXE_T / 2) + idx];
+      val[f][1] += val[f][0] >> 32;
+      o[f] = fma((double)val[f][1], 4294967296.0, (double)(val[f][0] & 0xffffffffll)) * sc * S.scale[f];
     }
   }
   /* algorithmic work of this unit (the same count as the FP64 kernel) */
@@ -302,11 +328,10 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
   if (tid < 32) {
     const long long msum = emask_products<DIM>(S.cnt, S.setup);
     if (tid > 0) return;
-    const double kphi = KER == KER_GAUSS ? 4.0 : 8.0;
-    const double fl = (double)pn * ((double)S.blk * (10.0 + kphi) + 2.0 * FP * (double)msum + NEN * (2.0 * FP + 1.0)) +
-                      18.0 * (double)S.wsum;
-    const double by = (double)pn * (8.0 * DIM + 4.0 + 8.0 * FP) + (double)S.blk * 8.0 * DIM + (double)msum * FP * 8.0;
-    atomicAdd(&P.ctrl->eval_flops, fl);
-    atomicAdd(&P.ctrl->eval_bytes, by);
+    const int kphi = KER == KER_GAUSS ? 4 : 8;
+    const long long fl = pn * ((long long)S.blk * (10 + kphi) + 2 * FP * msum + NEN * (2 * FP + 1)) + 18LL * S.wsum;
+    const long long by = (long long)pn * (8 * DIM + 4 + 8 * FP) + S.blk * 8LL * DIM + msum * FP * 8;
+    atomicAdd(&P.ctrl->eval_flops, (double)fl);
+    atomicAdd(&P.ctrl->eval_bytes, (double)by);
   }
 }

@@ -625,6 +625,7 @@ static int create_ctx(lgb_ctx **out)
   for (i = 0; i < 2 * NPROF; i++) cudaEventCreate(&c->ev[i]);
   c->launch_base = lgb_launch_count();
   d->chunk_cap = LGB_CHUNK_MAX;
+  d->unit_threads = 128;
   *out = c;
   return 0;
 }
@@ -942,9 +943,10 @@ static int fill_data(lgb_ctx *c, int n, const double *coords, const double *valu
    the largest of 128, 64 and 32 that gives every SM its four CTAs, so that small sets spread over the
    chip.
    FP32 record kernel (as many threads as the capacity up to 128, shared in the same way; 256: two
-   particles per thread): 128 threads for sets of so few units that the shares shorten the launch,
-   else the smallest of 32, 64 and 128 that holds a mean cell, so that units of sparse cells cost no
-   idle warps (1M particles of a mixture over 970,000 cells: 32 threads 4.0 ms per launch, 128 threads
+   particles per thread): 128 particles for sets of so few units that the shares shorten the launch, on
+   512 threads if the SMs hold one unit each, 256 for two (1,000 particles in 125 cells: 512 threads 27 us per launch, 128
+   40 us); else the smallest of 32, 64 and 128 that holds a mean cell, so that units of sparse cells cost no
+   idle warps (1M particles of a mixture over 970,000 cells: 32 threads 3.0 ms per launch, 128 threads
    23.5 ms).  From 128 particles per cell on, 128 or 256 by the warps their units keep busy, where
    two particles per thread cost 1.8 of one (563 per cell, 16.8M particles: 256 22.6 ms, 128 25.1 ms;
    144 per cell, 2M particles: 128 3.4 ms, 256 4.7 ms).
@@ -955,7 +957,7 @@ static double unit_warps(int n); /* warps that a unit of n <= 128 particles keep
 static int choose_chunk(lgb_ctx *c)
 {
   lgb_dev *d = &c->d;
-  int nc = d->g.ncells, i, m, cap = LGB_CHUNK_MAX;
+  int nc = d->g.ncells, i, m, cap = LGB_CHUNK_MAX, threads = 128;
   double bestcost = -1.0;
   const int fx = d->prec == LGB_PREC_FP32 ? d->F >= d->g.dim : d->fixed;
   const char *env = getenv("LAGRBF_CHUNK");
@@ -971,8 +973,10 @@ static int choose_chunk(lgb_ctx *c)
       n += cnt[i + 1] - cnt[i];
     }
     cap = 128;
-    if (units >= 4LL * d->nsm)
+    threads = units <= d->nsm ? 512 : units <= 2LL * d->nsm ? 256 : 128;
+    if (units >= 4LL * d->nsm) {
       for (cap = 32; cap < LGB_CHUNK_MAX && n > cap * used; cap *= 2) ;
+    }
     if (cap > 128) {
       double c1 = 0.0, c2 = 0.0;
       for (i = 0; i < nc; i++) {
@@ -982,7 +986,8 @@ static int choose_chunk(lgb_ctx *c)
       }
       if (c1 <= c2) cap = 128;
     }
-    if (!d->rec32 && cap < 64) cap = 64; /* gather kernel */
+    if (!d->rec32 && cap < 64) cap = 64; /* gather kernel, or no data yet */
+    if (cap < 128) threads = cap;
   } else if (fx) {
     for (cap = 128; cap > 32; cap /= 2) {
       long long units = 0;
@@ -1005,9 +1010,13 @@ static int choose_chunk(lgb_ctx *c)
     }
   }
   free(cnt);
-  if (env && (atoi(env) == 64 || atoi(env) == 128 || (atoi(env) == 256 && !(fx && d->prec != LGB_PREC_FP32)))) cap = atoi(env);
-  if (cap != d->chunk_cap) {
+  if (env && (atoi(env) == 64 || atoi(env) == 128 || (atoi(env) == 256 && !(fx && d->prec != LGB_PREC_FP32)))) {
+    cap = atoi(env);
+    threads = cap < 128 ? cap : 128;
+  }
+  if (cap != d->chunk_cap || threads != d->unit_threads) {
     d->chunk_cap = cap;
+    d->unit_threads = threads;
     invalidate_graph(c);
     OP(lgb_op_bin_particles(d, 0, c->stream)); /* chunk offsets for the new capacity */
   }

@@ -195,6 +195,7 @@ typedef struct {
   int *cell_p, *alive, *pcount, *pstart, *pfill, *plist, *chunk_start;
   int max_chunks;
   int chunk_cap;       /* particles per evaluation work unit */
+  int unit_threads;    /* threads of a work unit of the FP32 record kernel */
   /* precomputed FP32 record blocks streamed by TMA (NULL: gather staging) */
   float *rec32;
   long long *rec_off;
