@@ -3,6 +3,7 @@
  */
 #pragma once
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 #include <string.h>
 #include "lgb_internal.h"
@@ -27,20 +28,24 @@ __host__ __device__ __forceinline__ long long lgb_key(double v)
 /* Cell of a point on the uniform PU mesh (DMSwarmPICSetCellId / DMLocatePoints on a uniform DMDA,
    the convention the oracle fixes): -1 outside [O, L] or NaN, else per axis
    clamp(floor((x - O) / h), 0, n - 2) in FP64, x == L in the last cell.  With the face keys the same index is the number
-   of faces at or below x (integer binary search; the FP64 division and floor would keep GB300's
-   FP64 pipe, 1/64 of the FP32 rate, busy for the whole launch). */
-__device__ __forceinline__ int lgb_locate(const lgb_geom &g, const double *x)
+   of faces at or below x: an FP32 estimate, which the keys of its two faces confirm (independent loads),
+   else, next to a face, an integer binary search (dependent loads).  The FP64 division and floor would keep GB300's
+   FP64 pipe, 1/64 of the FP32 rate, busy for the whole launch. */
+template <int DIM>
+__device__ __forceinline__ int lgb_locate(const lgb_geom &g, const double (&x)[3])
 {
   int c[3] = {0, 0, 0};
 #pragma unroll
-  for (int d = 0; d < 3; d++) {
-    if (d >= g.dim) break;
-    double xd = x[d];
+  for (int d = 0; d < DIM; d++) {
+    const double xd = x[d];
     if (g.bkey) {
       const long long k = lgb_key(xd);
       if (k < g.okey[d] || k > g.lkey[d]) return -1;
       const long long *b = g.bkey + g.boff[d];
       int lo = 0, hi = g.n[d] - 2; /* faces b[0 .. n-3]; the answer is how many are <= k */
+      const int t = min(max((int)(((float)xd - (float)g.O[d]) * (float)g.rh[d]), lo), hi);
+      const long long below = t > lo ? __ldg(b + t - 1) : k, above = t < hi ? __ldg(b + t) : LLONG_MAX;
+      if (below <= k && k < above) lo = hi = t;
       while (lo < hi) {
         const int mid = (lo + hi) >> 1;
         if (__ldg(b + mid) <= k) lo = mid + 1; else hi = mid;
@@ -55,6 +60,12 @@ __device__ __forceinline__ int lgb_locate(const lgb_geom &g, const double *x)
     }
   }
   return c[0] + c[1] * g.nc[0] + c[2] * g.nc[0] * g.nc[1];
+}
+
+__device__ __forceinline__ int lgb_locate(const lgb_geom &g, const double *x)
+{
+  const double xi[3] = {x[0], x[1], g.dim == 3 ? x[2] : 0.0};
+  return g.dim == 3 ? lgb_locate<3>(g, xi) : lgb_locate<2>(g, xi);
 }
 
 __device__ __forceinline__ void lgb_cell_ijk(const lgb_geom &g, int cell, int &i, int &j, int &l)

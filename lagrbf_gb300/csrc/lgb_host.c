@@ -262,7 +262,7 @@ typedef struct lgb_ctx_s {
   void *ruser;
   /* graph of one internal step */
   cudaGraphExec_t graph;
-  int graph_valid, graph_mode; /* graph_mode: 1 when the captured step is analytical */
+  int graph_valid, graph_mode; /* graph_mode: 1 when the captured step is analytical, 2 without set-up */
   long long graph_launches, graph_eval_launches;
   /* the step inside a device-side while loop: one launch advances a whole advection interval */
   cudaGraphExec_t wgraph;
@@ -353,7 +353,7 @@ static void destroy_ctx(lgb_ctx *c)
   free_particles(d);
   DFREE(d->cstart); DFREE(d->dfill); DFREE(d->pm); DFREE(d->slot); DFREE(d->setup); DFREE(d->solved);
   DFREE(d->need); DFREE(d->work); DFREE(d->work_s); DFREE(d->cexp); DFREE(d->status); DFREE(d->coff); DFREE(d->foff); DFREE(d->c64); DFREE(d->kappa);
-  DFREE(d->c32); DFREE(d->fac); DFREE(d->ws); DFREE(d->pcount); DFREE(d->pstart); DFREE(d->pfill);
+  DFREE(d->c32); DFREE(d->fac); DFREE(d->ws); DFREE(d->pcount); DFREE(d->pstart); DFREE(d->scan_tiles);
   DFREE(d->chunk_start); DFREE(d->scan_tmp); DFREE(d->scan_tmp64); DFREE(d->ctrl);
   DFREE(d->rec32); DFREE(d->rec_off); DFREE(d->bkey_buf); DFREE(d->cls_off_dev); DFREE(d->cdirty);
   for (i = 0; i < 2 * NPROF; i++) if (c->ev[i]) cudaEventDestroy(c->ev[i]);
@@ -581,7 +581,7 @@ static int create_ctx(lgb_ctx **out)
   d->foff = (long long *)dalloc(sizeof(long long) * (size_t)(nn + 1), &err);
   d->pcount = (int *)dalloc(sizeof(int) * (size_t)(nc + 1), &err);
   d->pstart = (int *)dalloc(sizeof(int) * (size_t)(nc + 1), &err);
-  d->pfill = (int *)dalloc(sizeof(int) * (size_t)(nc + 1), &err);
+  d->scan_tiles = (int *)dalloc(sizeof(int) * 2 * ((size_t)nc / 4096 + 2), &err);
   d->chunk_start = (int *)dalloc(sizeof(int) * (size_t)(nc + 1), &err);
   d->cdirty = (unsigned char *)dalloc((size_t)nc, &err);
   d->scan_tmp = (int *)dalloc(sizeof(int) * 4096, &err);
@@ -602,6 +602,7 @@ static int create_ctx(lgb_ctx **out)
   cudaMemsetAsync(d->need, 0, sizeof(int) * 2 * (size_t)nn, c->stream);
   cudaMemsetAsync(d->cstart, 0, sizeof(int) * (size_t)(nc + 1), c->stream);
   cudaMemsetAsync(d->pstart, 0, sizeof(int) * (size_t)(nc + 1), c->stream);
+  cudaMemsetAsync(d->pcount, 0, sizeof(int) * (size_t)(nc + 1), c->stream);
   cudaMemsetAsync(d->chunk_start, 0, sizeof(int) * (size_t)(nc + 1), c->stream);
   cudaMemsetAsync(d->cdirty, 0, (size_t)nc, c->stream);
   memset(c->hctrl, 0, sizeof(lgb_ctrl));
@@ -1018,7 +1019,7 @@ static int choose_chunk(lgb_ctx *c)
     d->chunk_cap = cap;
     d->unit_threads = threads;
     invalidate_graph(c);
-    OP(lgb_op_bin_particles(d, 0, c->stream)); /* chunk offsets for the new capacity */
+    OP(lgb_op_bin_particles(d, c->stream)); /* chunk offsets for the new capacity */
   }
   d->max_chunks = d->g.ncells + (d->np + d->chunk_cap - 1) / d->chunk_cap + 1;
   return 0;
@@ -1093,7 +1094,7 @@ static int fill_points(lgb_ctx *c, int n, const double *coords, const double *va
     if (e != cudaSuccess)
       return set_error(LAGRBF_ERR_GPU, "copying the particles to the device failed: %s", cudaGetErrorString(e));
   }
-  OP(lgb_op_bin_particles(d, 1, c->stream));
+  OP(lgb_op_bin_particles(d, c->stream));
   TRY(choose_chunk(c));
   CU(cudaStreamSynchronize(c->stream));
   c->points_filled = 1;
@@ -1134,9 +1135,17 @@ static int eval_fields(lgb_ctx *c, int nf_first, int nf, double *out, int stride
   return 0;
 }
 
+/* Option setup_all_patches after an interpolation: every patch is set up and solved for the current data
+   (of the owner, when they are borrowed), and nothing would be queued. */
+static int nothing_to_set_up(const lgb_ctx *c)
+{
+  return c->d.setup_all && (c->shared_from ? c->shared_from->all_ready : c->all_ready);
+}
+
 /* LagRBF_PartitionsSetUp: queue the patches touched by live particles, set up / solve them. */
 static int partitions_setup(lgb_ctx *c)
 {
+  if (nothing_to_set_up(c)) return 0;
   OP(lgb_op_mark_patches(&c->d, c->stream));
   if (c->profiling) {
     prof_collect(c, &c->eval_ms);
@@ -1220,51 +1229,55 @@ static int eval_velocity(lgb_ctx *c, int analytical)
   return eval_fields(c, 0, c->d.g.dim, c->d.vel, c->d.g.dim);
 }
 
-/* One internal step of InternalForwardAdvectionLoop after the dt selection. */
-static int step_sequence(lgb_ctx *c, int analytical)
+/* One internal step of InternalForwardAdvectionLoop; loop: the conditional handle when the step is the body
+   of the device-side loop, whose condition kernel ends a step and begins the next. */
+static int step_sequence(lgb_ctx *c, int analytical, const unsigned long long *loop)
 {
   lgb_dev *d = &c->d;
   void *s = c->stream;
   int st;
   const int pp = (c->scheme == LGB_DOPRI && d->dopri_pp);
-  OP(lgb_op_ctrl(d, pp ? LGB_CTRL_BEGIN_SWEEP : LGB_CTRL_BEGIN_STEP, s));
+  /* a device-side analytical velocity is evaluated particle by particle: the cells' lists only after the step */
+  const int bin = !(analytical && d->vfield);
+  if (!loop) OP(lgb_op_ctrl(d, pp ? LGB_CTRL_BEGIN_SWEEP : LGB_CTRL_BEGIN_STEP, s));
   switch (c->scheme) {
   case LGB_RK1:
-    OP(lgb_op_stage(d, LGB_RK1, 0, s));
-    OP(lgb_op_bin_particles(d, 1, s));
+    OP(lgb_op_stage(d, LGB_RK1, 0, 1, s));
+    OP(lgb_op_bin_located(d, NULL, s));
     break;
   case LGB_RK2:
-    OP(lgb_op_stage(d, LGB_RK2, 0, s));
-    OP(lgb_op_bin_particles(d, 1, s));
+    OP(lgb_op_stage(d, LGB_RK2, 0, bin, s));
+    if (bin) OP(lgb_op_bin_located(d, NULL, s));
     TRY(eval_velocity(c, analytical));
-    OP(lgb_op_stage(d, LGB_RK2, 1, s));
-    OP(lgb_op_bin_particles(d, 1, s));
+    OP(lgb_op_stage(d, LGB_RK2, 1, 1, s));
+    OP(lgb_op_bin_located(d, NULL, s));
     break;
   case LGB_RK4:
     for (st = 0; st < 3; st++) {
-      OP(lgb_op_stage(d, LGB_RK4, st, s));
-      OP(lgb_op_bin_particles(d, 1, s));
+      OP(lgb_op_stage(d, LGB_RK4, st, bin, s));
+      if (bin) OP(lgb_op_bin_located(d, NULL, s));
       TRY(eval_velocity(c, analytical));
     }
-    OP(lgb_op_stage(d, LGB_RK4, 3, s));
-    OP(lgb_op_bin_particles(d, 1, s));
+    OP(lgb_op_stage(d, LGB_RK4, 3, 1, s));
+    OP(lgb_op_bin_located(d, NULL, s));
     break;
   case LGB_DOPRI:
     if (pp) {
       /* per-particle steps: only the particles still short of t_next are staged and evaluated */
       OP(lgb_op_pp_begin(d, s));
       for (st = 0; st < 6; st++) {
-        OP(lgb_op_stage(d, LGB_DOPRI, st, s));
-        OP(lgb_op_bin_particles_mask(d, 1, d->active, s));
+        OP(lgb_op_stage(d, LGB_DOPRI, st, bin, s));
+        if (bin) OP(lgb_op_bin_located(d, d->active, s));
         TRY(eval_velocity(c, analytical));
       }
       OP(lgb_op_pp_accept(d, s));
-      OP(lgb_op_bin_particles(d, 1, s)); /* rejected particles are back at x0 */
+      OP(lgb_op_bin_particles(d, s)); /* rejected particles are back at x0 */
       break;
     }
     for (st = 0; st < 6; st++) {
-      OP(lgb_op_stage(d, LGB_DOPRI, st, s));
-      OP(lgb_op_bin_particles(d, 1, s));
+      const int b = bin || st == 5;
+      OP(lgb_op_stage(d, LGB_DOPRI, st, b, s));
+      if (b) OP(lgb_op_bin_located(d, NULL, s));
       TRY(eval_velocity(c, analytical));
     }
     OP(lgb_op_dopri_error(d, s));
@@ -1276,14 +1289,15 @@ static int step_sequence(lgb_ctx *c, int analytical)
   if (!analytical) {
     TRY(partitions_setup(c));
     if (d->F > 0) TRY(eval_fields(c, 0, d->F, d->fields, d->F));
-    OP(lgb_op_ctrl(d, LGB_CTRL_RESET_CFL, s));
     OP(lgb_op_copy_velocity(d, s));
   } else {
     TRY(host_velocity(c));
-    OP(lgb_op_ctrl(d, LGB_CTRL_RESET_CFL, s));
     OP(lgb_op_count_alive(d, s));
   }
-  OP(lgb_op_ctrl(d, pp ? LGB_CTRL_END_SWEEP : LGB_CTRL_END_STEP, s));
+  if (loop)
+    OP(lgb_op_loop_cond(d, pp ? LGB_CTRL_END_SWEEP : LGB_CTRL_END_STEP,
+                        pp ? LGB_CTRL_BEGIN_SWEEP : LGB_CTRL_BEGIN_STEP, *loop, s));
+  else OP(lgb_op_ctrl(d, pp ? LGB_CTRL_END_SWEEP : LGB_CTRL_END_STEP, s));
   return 0;
 }
 
@@ -1322,10 +1336,11 @@ static int couple_ranks(lgb_ctx *c, int dopri_update)
 static int run_step(lgb_ctx *c, int analytical)
 {
   /* the captured step differs between interpolated and device-field analytical advection */
-  if (c->graph_valid && c->graph_mode != analytical) invalidate_graph(c);
+  const int mode = analytical ? 1 : nothing_to_set_up(c) ? 2 : 0;
+  if (c->graph_valid && c->graph_mode != mode) invalidate_graph(c);
   if ((analytical && !c->d.vfield) || c->profiling || !c->use_graph) {
     long long l0 = lgb_launch_count();
-    TRY(step_sequence(c, analytical));
+    TRY(step_sequence(c, analytical, NULL));
     c->launches_graph += 0;
     (void)l0;
     prof_collect(c, &c->eval_ms);
@@ -1339,7 +1354,7 @@ static int run_step(lgb_ctx *c, int analytical)
     cudaError_t e = cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal);
     int rc = 0;
     if (e == cudaSuccess) {
-      rc = step_sequence(c, analytical);
+      rc = step_sequence(c, analytical, NULL);
       e = cudaStreamEndCapture(c->stream, &graph);
     }
     c->graph_eval_launches = c->eval_launches - e0;
@@ -1348,17 +1363,17 @@ static int run_step(lgb_ctx *c, int analytical)
       /* capture not possible: run this step eagerly and stop using graphs */
       cudaGetLastError();
       c->use_graph = 0;
-      TRY(step_sequence(c, analytical));
+      TRY(step_sequence(c, analytical, NULL));
     } else {
       e = cudaGraphInstantiate(&c->graph, graph, 0);
       cudaGraphDestroy(graph);
       if (e != cudaSuccess) {
         cudaGetLastError();
         c->use_graph = 0;
-        TRY(step_sequence(c, analytical));
+        TRY(step_sequence(c, analytical, NULL));
       } else {
         c->graph_valid = 1;
-        c->graph_mode = analytical;
+        c->graph_mode = mode;
         c->graph_launches = lgb_launch_count() - l0;
         /* the captured launches did not run; count them when the graph replays */
         c->launch_base += c->graph_launches;
@@ -1376,7 +1391,7 @@ static int run_step(lgb_ctx *c, int analytical)
   return 0;
 }
 
-static int step_sequence(lgb_ctx *c, int analytical);
+static int step_sequence(lgb_ctx *c, int analytical, const unsigned long long *loop);
 
 /* The internal steps of one advection interval as one graph launch: the step is the body of a
    conditional while node whose condition kernel continues while t < t_next (and no error flag is
@@ -1386,11 +1401,12 @@ static int step_sequence(lgb_ctx *c, int analytical);
 static int run_interval_on_device(lgb_ctx *c, int analytical, int *rc)
 {
   long long s0;
+  const int mode = analytical ? 1 : nothing_to_set_up(c) ? 2 : 0;
   *rc = 0;
   if (!c->use_graph || !c->device_loop || c->profiling || c->reduce || (analytical && !c->d.vfield) ||
       c->wgraph_failed)
     return 0;
-  if (c->wgraph_valid && c->wgraph_mode != analytical) invalidate_graph(c);
+  if (c->wgraph_valid && c->wgraph_mode != mode) invalidate_graph(c);
   if (!c->wgraph_valid) {
     cudaGraph_t g = NULL, body;
     cudaGraphConditionalHandle h;
@@ -1412,8 +1428,8 @@ static int run_interval_on_device(lgb_ctx *c, int analytical, int *rc)
       ok = cudaStreamBeginCaptureToGraph(c->stream, body, NULL, NULL, 0, cudaStreamCaptureModeThreadLocal) ==
            cudaSuccess;
       if (ok) {
-        int r = step_sequence(c, analytical);
-        if (!r) r = lgb_op_loop_cond(&c->d, (unsigned long long)h, c->stream);
+        const unsigned long long hh = (unsigned long long)h;
+        int r = step_sequence(c, analytical, &hh);
         ok = (cudaStreamEndCapture(c->stream, &body) == cudaSuccess) && !r;
         /* a capture into the conditional body that failed leaves that body in no defined state:
            destroying the parent graph then crashed the driver, so this one graph is left alone
@@ -1433,9 +1449,11 @@ static int run_interval_on_device(lgb_ctx *c, int analytical, int *rc)
       return 0;
     }
     c->wgraph_valid = 1;
-    c->wgraph_mode = analytical;
+    c->wgraph_mode = mode;
   }
   s0 = c->hctrl->steps;
+  /* the loop's steps begin in the condition kernel of the step before */
+  OP(lgb_op_ctrl(&c->d, (c->scheme == LGB_DOPRI && c->d.dopri_pp) ? LGB_CTRL_BEGIN_SWEEP : LGB_CTRL_BEGIN_STEP, c->stream));
   CU(cudaGraphLaunch(c->wgraph, c->stream));
   CU(cudaMemcpyAsync(c->hctrl, c->d.ctrl, sizeof(lgb_ctrl), cudaMemcpyDeviceToHost, c->stream));
   CU(cudaStreamSynchronize(c->stream));

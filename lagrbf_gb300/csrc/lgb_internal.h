@@ -129,14 +129,16 @@ typedef struct {
   long long particle_steps;
   double eval_flops;   /* accumulated algorithmic flops of evaluation launches   */
   double eval_bytes;   /* accumulated algorithmic bytes of evaluation launches   */
-  int nwork;           /* patches queued for set-up / solve                       */
+  /* cleared together before every queueing: patches queued for set-up / solve, the queued patches of
+     each size class (the class work lists) and the next entry of each list, the same of the patches
+     that only re-solve */
+  int nwork;
+  int nwork_c[LGB_NCLS], next_c[LGB_NCLS];
+  int nwork_s[LGB_NCLS], next_s[LGB_NCLS];
   int factor_error;    /* first non-positive pivot row (1-based), 0 if none        */
   int factor_node;     /* patch with that pivot                                    */
   int nfactored;
   double factor_flops;
-  int nwork_c[LGB_NCLS];  /* queued patches of each size class (the class work lists)      */
-  int next_c[LGB_NCLS];   /* next entry of each class's work list (blocked factorisation)  */
-  int nwork_s[LGB_NCLS], next_s[LGB_NCLS]; /* the same of the patches that only re-solve        */
   int eval_error;      /* a bounded wait of the evaluation kernel gave up */
   int pp_left;         /* per-particle Dormand-Prince: particles still short of t_next   */
   double dt_cfl_ext;   /* > 0: the CFL step agreed over ranks (replaces the local one)     */
@@ -192,7 +194,8 @@ typedef struct {
   /* particle swarm */
   int np, np_cap;
   double *xp, *fields, *vel, *x0, *vadv;
-  int *cell_p, *alive, *pcount, *pstart, *pfill, *plist, *chunk_start;
+  int *cell_p, *alive, *pcount, *pstart, *plist, *chunk_start; /* pcount: zero between binnings */
+  int *scan_tiles;     /* tile sums of the two binning scans (2 ints per tile) */
   int max_chunks;
   int chunk_cap;       /* particles per evaluation work unit */
   int unit_threads;    /* threads of a work unit of the FP32 record kernel */
@@ -223,12 +226,13 @@ int lgb_op_locate(const lgb_geom *g, int n, const double *x, int *cell, int *ali
                   void *stream);
 int lgb_op_scan_i32(int n, const int *in, int *out, int *tmp, void *stream);
 int lgb_op_scan_i64(int n, const long long *in, long long *out, long long *tmp, void *stream);
-int lgb_op_scatter(int n, const int *cell, const int *alive, const int *start, int *fill, int *list, void *stream);
+int lgb_op_scatter(int n, const int *cell, const int *start, int *fill, int *list, void *stream);
 int lgb_op_data_arrange(lgb_dev *d, void *stream);      /* xs, xr, fs, patch sizes, slots, offsets */
 int lgb_op_data_values(lgb_dev *d, void *stream);       /* fs only (values changed)                */
-int lgb_op_bin_particles(lgb_dev *d, int mark_dead, void *stream); /* cell_p, pcount, pstart, plist, chunks */
-/* the same, listing for evaluation only the particles with active[p] != 0 (all are located) */
-int lgb_op_bin_particles_mask(lgb_dev *d, int mark_dead, const int *active, void *stream);
+/* cell_p, pstart, plist, chunk_start; particles that left the domain are removed */
+int lgb_op_bin_particles(lgb_dev *d, void *stream);
+/* the lists and work units of particles that lgb_op_stage has located and counted (active: its mask) */
+int lgb_op_bin_located(lgb_dev *d, const int *active, void *stream);
 int lgb_op_mark_patches(lgb_dev *d, void *stream);      /* queue patches touched by live particles */
 /* lgb_factor.cu */
 int lgb_op_factor(lgb_dev *d, void *stream);            /* set up / solve queued patches */
@@ -237,7 +241,7 @@ int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int out_stride, v
 int lgb_op_weights(lgb_dev *d, double *w, void *stream);
 int lgb_op_build_records(lgb_dev *d, int force, void *stream);
 /* lgb_step.cu */
-int lgb_op_stage(lgb_dev *d, int scheme, int stage, void *stream);
+int lgb_op_stage(lgb_dev *d, int scheme, int stage, int bin, void *stream); /* positions, cell_p; bin: count for lgb_op_bin_located */
 int lgb_op_dopri_error(lgb_dev *d, void *stream);
 int lgb_op_ctrl(lgb_dev *d, int what, void *stream);
 enum { LGB_CTRL_BEGIN_STEP = 0, LGB_CTRL_END_STEP = 1, LGB_CTRL_RESET_CFL = 2, LGB_CTRL_DOPRI_DT = 3,
@@ -248,10 +252,11 @@ int lgb_op_pp_init(lgb_dev *d, double t, void *stream);
 int lgb_op_pp_begin(lgb_dev *d, void *stream);
 int lgb_op_pp_accept(lgb_dev *d, void *stream);
 int lgb_op_copy_velocity(lgb_dev *d, void *stream);     /* vel <- fields[:, :dim] */
-/* Condition of the device-side step loop (a conditional while node of the step graph, handle =
-   a cudaGraphConditionalHandle): continue while t < t_next, no error flag is set and the
-   iteration limit is not reached. */
-int lgb_op_loop_cond(lgb_dev *d, unsigned long long handle, void *stream);
+/* The end of a step (LGB_CTRL_END_*), the condition of the device-side step loop (a conditional while
+   node of the step graph, handle = a cudaGraphConditionalHandle): continue while t < t_next, no error
+   flag is set and the iteration limit is not reached; and, when it continues, the beginning of the
+   next step (LGB_CTRL_BEGIN_*). */
+int lgb_op_loop_cond(lgb_dev *d, int end, int begin, unsigned long long handle, void *stream);
 int lgb_op_count_alive(lgb_dev *d, void *stream);
 int lgb_op_velocity_field(lgb_dev *d, void *stream);    /* vel <- analytical field at live particles */
 int lgb_device_info(int *nsm, int *smem_optin);

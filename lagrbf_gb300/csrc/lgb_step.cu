@@ -7,7 +7,7 @@
  * (advection.c:298-316) and the loop scalars of InternalForwardAdvectionLoop (time_loop.c:39-100).
  *
  * Every stage is one pass over the particles that writes the stage position (and commits the
- * previous stage velocity into v_adv), followed by re-binning and one evaluation.  The global
+ * previous stage velocity into v_adv) and locates it, followed by the cells' lists and one evaluation.  The global
  * reductions of the reference (CFL min dt, DOPRI max error: MPI_Allreduce sites advection.c:466,
  * dormand_prince.c:93) are warp-reduced atomics on the ordered bit patterns of non-negative
  * doubles.  The loop scalars (t, dt, DOPRI dt) live in a device control block, so a whole
@@ -28,9 +28,17 @@ __constant__ double c_dp_e[7] = {5179.0 / 57600.0, 0, 7571.0 / 16695.0, 393.0 / 
                                  187.0 / 2100.0, 1.0 / 40.0};
 
 /* AdvectionProjectOntoSphereBoundary_Pointwise (advection.c:472-491) */
-__device__ __forceinline__ void project_sphere(double *x, int dim, double rmin, double rmax)
+template <int dim>
+__device__ __forceinline__ void project_sphere(double *x, double rmin, double rmax)
 {
   double pos = 0.0, normal[3];
+  /* rmin = 0 and rmax^2 = inf (the defaults): nothing to do where 0 < |x|^2 < inf, which the exponent of the
+     largest component shows without the FP64 pipe */
+  if (__double2hiint(rmax) >= 0x5ff00000 && __double2hiint(rmax) < 0x7ff00000 && __double_as_longlong(rmin) == 0) {
+    int m = 0;
+    for (int d = 0; d < dim; d++) m = max(m, __double2hiint(x[d]) & 0x7fffffff);
+    if (m >= 0x20b00000 && m < 0x5fd00000) return; /* 2^-500 <= max |x_d| < 2^510 */
+  }
   for (int d = 0; d < dim; d++) pos += x[d] * x[d];
   if (pos < rmax * rmax && pos > rmin * rmin) return;
   pos = sqrt(pos);
@@ -40,36 +48,37 @@ __device__ __forceinline__ void project_sphere(double *x, int dim, double rmin, 
 }
 
 struct StageParams {
-  int np, dim, scheme, stage;
+  int np, scheme, stage;
   double *xp, *x0, *vel, *vadv;
-  const int *alive;
+  int *alive;
   const lgb_ctrl *ctrl;
+  lgb_geom g;
+  int *cell;           /* cell of the new position */
+  int *counts;         /* particles per cell (NULL: not binned) */
   const double *hcur;  /* per-particle Dormand-Prince: the particle's step (else NULL: ctrl->dt) */
   const int *active;   /* per-particle Dormand-Prince: particles taking part in the sweep      */
 };
 
-__global__ void k_stage(StageParams S)
+/* The position after the stage, in xs (and S.xp). */
+template <int dim>
+__device__ __forceinline__ void stage_position(const StageParams &S, int p, double (&xs)[3])
 {
-  int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= S.np || !S.alive[p]) return;
-  if (S.active && !S.active[p]) return;
-  const int dim = S.dim;
   const double dt = S.hcur ? S.hcur[p] : S.ctrl->dt;
   const double rmin = S.ctrl->rmin, rmax = S.ctrl->rmax;
   const size_t o = (size_t)p * dim;
   const size_t st = (size_t)S.np * dim; /* stride between v_adv stages */
-  double x[3], x0[3], v[3];
+  double x[3], x0[3], v[3]; /* dim of each are used, in registers: the loops unroll */
   for (int d = 0; d < dim; d++) { x[d] = S.xp[o + d]; v[d] = S.vel[o + d]; }
   switch (S.scheme) {
   case LGB_RK1:
     /* runge_kutta_1.c:61-64: x = x0 + dt * v */
-    for (int d = 0; d < dim; d++) S.xp[o + d] = x[d] + dt * v[d];
+    for (int d = 0; d < dim; d++) S.xp[o + d] = xs[d] = x[d] + dt * v[d];
     return;
   case LGB_RK2:
     if (S.stage == 0) {
-      for (int d = 0; d < dim; d++) { S.x0[o + d] = x[d]; S.xp[o + d] = x[d] + (0.5 * dt) * v[d]; }
+      for (int d = 0; d < dim; d++) { S.x0[o + d] = x[d]; S.xp[o + d] = xs[d] = x[d] + (0.5 * dt) * v[d]; }
     } else {
-      for (int d = 0; d < dim; d++) S.xp[o + d] = S.x0[o + d] + dt * v[d];
+      for (int d = 0; d < dim; d++) S.xp[o + d] = xs[d] = S.x0[o + d] + dt * v[d];
     }
     return;
   case LGB_RK4: {
@@ -80,19 +89,18 @@ __global__ void k_stage(StageParams S)
     for (int d = 0; d < dim; d++) S.vadv[S.stage * st + o + d] = v[d];
     if (S.stage == 0) for (int d = 0; d < dim; d++) S.x0[o + d] = x0[d];
     if (S.stage < 3) {
-      double xs[3];
       for (int d = 0; d < dim; d++) xs[d] = x0[d] + (c[S.stage] * dt) * v[d];
-      project_sphere(xs, dim, rmin, rmax);
+      project_sphere<dim>(xs, rmin, rmax);
       for (int d = 0; d < dim; d++) S.xp[o + d] = xs[d];
     } else {
       const double w[4] = {1.0, 2.0, 2.0, 1.0};
-      double xs[3];
       for (int d = 0; d < dim; d++) xs[d] = x[d]; /* components not yet updated keep the stage-3 value */
+#pragma unroll
       for (int d = 0; d < dim; d++) {
         double sum = 0.0;
         for (int s = 0; s < 4; s++) sum += w[s] * S.vadv[s * st + o + d];
         xs[d] = x0[d] + dt / 6.0 * sum;
-        project_sphere(xs, dim, rmin, rmax); /* runge_kutta_4.c:140, inside the component loop */
+        project_sphere<dim>(xs, rmin, rmax); /* runge_kutta_4.c:140, inside the component loop */
       }
       for (int d = 0; d < dim; d++) S.xp[o + d] = xs[d];
     }
@@ -103,14 +111,15 @@ __global__ void k_stage(StageParams S)
     if (s == 0) for (int d = 0; d < dim; d++) { x0[d] = x[d]; S.x0[o + d] = x[d]; }
     else for (int d = 0; d < dim; d++) x0[d] = S.x0[o + d];
     for (int d = 0; d < dim; d++) S.vadv[s * st + o + d] = v[d];
-    double vs[3] = {0.0, 0.0, 0.0}, xs[3];
+    double vs[3] = {0.0, 0.0, 0.0};
     for (int j = 0; j <= s; j++)
+#pragma unroll
       for (int d = 0; d < dim; d++) {
         double vj = (j == s) ? v[d] : S.vadv[j * st + o + d];
         vs[d] += c_dp_a[s][j] * vj;
       }
     for (int d = 0; d < dim; d++) { S.vel[o + d] = vs[d]; xs[d] = x0[d] + dt * vs[d]; }
-    project_sphere(xs, dim, rmin, rmax);
+    project_sphere<dim>(xs, rmin, rmax);
     for (int d = 0; d < dim; d++) S.xp[o + d] = xs[d];
     return;
   }
@@ -118,23 +127,46 @@ __global__ void k_stage(StageParams S)
   }
 }
 
-extern "C" int lgb_op_stage(lgb_dev *d, int scheme, int stage, void *stream)
+/* One stage of one particle per thread.  The new position is located at once instead of being read back
+   by a kernel of its own; what left the domain is removed (DMSwarmMigrate on one rank).  Particles without a
+   part in the stage stay where they were located.  4M particles in 2D, four RK4 stages with their
+   locating: 0.96 ms before, 0.60 now. */
+template <int DIM>
+__global__ void k_stage(StageParams S)
+{
+  int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= S.np || !S.alive[p]) return;
+  if (S.active && !S.active[p]) return;
+  double xs[3];
+  stage_position<DIM>(S, p, xs);
+  const int c = lgb_locate<DIM>(S.g, xs);
+  S.cell[p] = c;
+  if (c < 0) S.alive[p] = 0;
+  else if (S.counts) atomicAdd(&S.counts[c], 1);
+}
+
+extern "C" int lgb_op_stage(lgb_dev *d, int scheme, int stage, int bin, void *stream)
 {
   if (d->np <= 0) return 0;
   StageParams S;
-  S.np = d->np; S.dim = d->g.dim; S.scheme = scheme; S.stage = stage;
+  S.np = d->np; S.scheme = scheme; S.stage = stage;
   S.xp = d->xp; S.x0 = d->x0; S.vel = d->vel; S.vadv = d->vadv; S.alive = d->alive; S.ctrl = d->ctrl;
   const int pp = (scheme == LGB_DOPRI && d->dopri_pp);
   S.hcur = pp ? d->hcur : NULL;
   S.active = pp ? d->active : NULL;
-  k_stage<<<lgb_cdiv(d->np, 256), 256, 0, (cudaStream_t)stream>>>(S);
+  S.g = d->g;
+  S.cell = d->cell_p;
+  S.counts = bin ? d->pcount : NULL;
+  if (d->g.dim == 3) k_stage<3><<<lgb_cdiv(d->np, 256), 256, 0, (cudaStream_t)stream>>>(S);
+  else k_stage<2><<<lgb_cdiv(d->np, 256), 256, 0, (cudaStream_t)stream>>>(S);
   lgb_count_launch(1);
   return (int)cudaGetLastError();
 }
 
 /* DOPRI embedded error (dormand_prince.c:37-102): commits v_adv_6, per-particle error norm,
    global max. */
-__global__ void k_dopri_error(int np, int dim, const double *__restrict__ xp, const double *__restrict__ x0,
+template <int dim>
+__global__ void k_dopri_error(int np, const double *__restrict__ xp, const double *__restrict__ x0,
                               const double *__restrict__ vel, double *__restrict__ vadv,
                               const int *__restrict__ alive, lgb_ctrl *ctrl)
 {
@@ -176,8 +208,10 @@ __global__ void k_dopri_error(int np, int dim, const double *__restrict__ xp, co
 extern "C" int lgb_op_dopri_error(lgb_dev *d, void *stream)
 {
   if (d->np <= 0) return 0;
-  k_dopri_error<<<lgb_cdiv(d->np, 256), 256, 0, (cudaStream_t)stream>>>(d->np, d->g.dim, d->xp, d->x0, d->vel,
-                                                                          d->vadv, d->alive, d->ctrl);
+  const int grid = lgb_cdiv(d->np, 256);
+  cudaStream_t s = (cudaStream_t)stream;
+  if (d->g.dim == 3) k_dopri_error<3><<<grid, 256, 0, s>>>(d->np, d->xp, d->x0, d->vel, d->vadv, d->alive, d->ctrl);
+  else k_dopri_error<2><<<grid, 256, 0, s>>>(d->np, d->xp, d->x0, d->vel, d->vadv, d->alive, d->ctrl);
   lgb_count_launch(1);
   return (int)cudaGetLastError();
 }
@@ -410,15 +444,22 @@ __global__ void k_velocity_field(int np, int dim, const double *__restrict__ x, 
     break;
   case LGB_VF_CELLULAR: {
     const double kx = par[1] * M_PI * X, ky = par[1] * M_PI * Y;
-    o[0] = par[0] * sin(kx) * cos(ky);
-    o[1] = -par[0] * cos(kx) * sin(ky);
+    double sx, cx, sy, cy;
+    sincos(kx, &sx, &cx); /* one argument reduction for both; the kernel is bound by the FP64 pipe */
+    sincos(ky, &sy, &cy);
+    o[0] = par[0] * sx * cy;
+    o[1] = -par[0] * cx * sy;
     break;
   }
   case LGB_VF_ABC: {
     const double a = par[3] * X, b = par[3] * Y, c = par[3] * Z;
-    o[0] = par[0] * sin(c) + par[2] * cos(b);
-    o[1] = par[1] * sin(a) + par[0] * cos(c);
-    o[2] = par[2] * sin(b) + par[1] * cos(a);
+    double sa, ca, sb, cb, sc, cc;
+    sincos(a, &sa, &ca);
+    sincos(b, &sb, &cb);
+    sincos(c, &sc, &cc);
+    o[0] = par[0] * sc + par[2] * cb;
+    o[1] = par[1] * sa + par[0] * cc;
+    o[2] = par[2] * sb + par[1] * ca;
     break;
   }
   case LGB_VF_FOURIER: {
@@ -447,7 +488,7 @@ extern "C" int lgb_op_velocity_field(lgb_dev *d, void *stream)
 }
 
 /* Loop scalars of InternalForwardAdvectionLoop, one thread. */
-__global__ void k_ctrl(lgb_ctrl *c, int what)
+__device__ void ctrl_op(lgb_ctrl *c, int what)
 {
   switch (what) {
   case LGB_CTRL_RESET_CFL:
@@ -467,6 +508,8 @@ __global__ void k_ctrl(lgb_ctrl *c, int what)
     c->dt_adv = dt; /* LagRBFSetTimeStep */
     c->maxerr_bits = 0ull;
     c->any_alive = 0;
+    c->n2max_bits = 0ull; /* for the velocity at the end of this step */
+    c->np_alive = 0;
     break;
   }
   case LGB_CTRL_DOPRI_DT: {
@@ -487,6 +530,8 @@ __global__ void k_ctrl(lgb_ctrl *c, int what)
     break;
   case LGB_CTRL_BEGIN_SWEEP:
     c->pp_left = 0;
+    c->n2max_bits = 0ull;
+    c->np_alive = 0;
     break;
   case LGB_CTRL_END_SWEEP: /* accepted particle steps are counted by k_pp_accept */
     if (c->pp_left == 0) c->t = c->t_next;
@@ -496,16 +541,20 @@ __global__ void k_ctrl(lgb_ctrl *c, int what)
   }
 }
 
-__global__ void k_loop_cond(lgb_ctrl *c, cudaGraphConditionalHandle h)
+__global__ void k_ctrl(lgb_ctrl *c, int what) { ctrl_op(c, what); }
+
+__global__ void k_loop_cond(lgb_ctrl *c, int end, int begin, cudaGraphConditionalHandle h)
 {
+  ctrl_op(c, end);
   c->loop_iter += 1;
   const int go = c->t < c->t_next && !c->factor_error && !c->eval_error && c->loop_iter < c->loop_cap;
+  if (go) ctrl_op(c, begin);
   cudaGraphSetConditional(h, go ? 1u : 0u);
 }
 
-extern "C" int lgb_op_loop_cond(lgb_dev *d, unsigned long long handle, void *stream)
+extern "C" int lgb_op_loop_cond(lgb_dev *d, int end, int begin, unsigned long long handle, void *stream)
 {
-  k_loop_cond<<<1, 1, 0, (cudaStream_t)stream>>>(d->ctrl, (cudaGraphConditionalHandle)handle);
+  k_loop_cond<<<1, 1, 0, (cudaStream_t)stream>>>(d->ctrl, end, begin, (cudaGraphConditionalHandle)handle);
   lgb_count_launch(1);
   return (int)cudaGetLastError();
 }
