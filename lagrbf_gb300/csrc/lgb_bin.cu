@@ -474,6 +474,21 @@ extern "C" int lgb_op_bin_located(lgb_dev *d, const int *active, void *stream)
   return 0;
 }
 
+__global__ void k_set_alive(int n, int *__restrict__ alive)
+{
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) alive[i] = 1;
+}
+
+extern "C" int lgb_op_set_alive(lgb_dev *d, void *stream)
+{
+  if (d->np <= 0) return 0;
+  k_set_alive<<<lgb_cdiv(d->np, 256), 256, 0, (cudaStream_t)stream>>>(d->np, d->alive);
+  lgb_count_launch(1);
+  LGB_CHECK_LAUNCH();
+  return 0;
+}
+
 extern "C" int lgb_op_bin_particles(lgb_dev *d, void *stream)
 {
   cudaStream_t s = (cudaStream_t)stream;

@@ -60,8 +60,8 @@ __device__ __forceinline__ long long fxe_phi(long long dx, long long dy, long lo
 }
 
 /* S w / 2^(64 - FXE_FINE), rounded, for a sum |S| < 2^61 and a weight w < 2^63.  The Gaussian kernel's sums cancel more:
-   three bits finer (relative error of a field against long double, 2D, 350 points per patch: 2.6e-16; FP64
-   3.2e-16; without them 3.9e-16; Wendland C2 2.2e-13 without, FP64 6.0e-13). */
+   three bits finer (relative error of a field against long double, 2D, 350 points per patch: 2.2e-16; FP64
+   3.2e-16; without them 3.9e-16; Wendland C2 2.0e-13 without, FP64 6.1e-13). */
 template <int KER> constexpr int fxe_fine = KER == KER_GAUSS ? 3 : 0;
 template <int KER>
 __device__ __forceinline__ long long fxe_weigh(long long s, unsigned long long w)

@@ -231,6 +231,7 @@ int lgb_op_data_arrange(lgb_dev *d, void *stream);      /* xs, xr, fs, patch siz
 int lgb_op_data_values(lgb_dev *d, void *stream);       /* fs only (values changed)                */
 /* cell_p, pstart, plist, chunk_start; particles that left the domain are removed */
 int lgb_op_bin_particles(lgb_dev *d, void *stream);
+int lgb_op_set_alive(lgb_dev *d, void *stream); /* every particle is in the domain */
 /* the lists and work units of particles that lgb_op_stage has located and counted (active: its mask) */
 int lgb_op_bin_located(lgb_dev *d, const int *active, void *stream);
 int lgb_op_mark_patches(lgb_dev *d, void *stream);      /* queue patches touched by live particles */
