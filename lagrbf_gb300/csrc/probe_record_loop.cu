@@ -2,10 +2,11 @@
  * probe_record_loop.cu -- compute-only bound of the FP32 record loop of k_eval_rec (not part of the
  * library; built and run by lagrbf_gb300/probe_eval.py).
  *
- * The loop body of lgb_evalrec.cuh (packed FP32 pairs: distance, rsqrt, Wendland C2 polynomial,
+ * The packed FP32 operations of the loop body of lgb_evalrec.cuh, there on pairs of points, here on pairs of
+ * particles against records that hold every value twice, with a minimum in place of the saturating FMA (distance, rsqrt, Wendland C2 polynomial,
  * per-patch FMAs for three fields and NI = 1, 2, 4 involved patches) runs over a block of records
  * held in shared memory for the whole kernel: no staging, no prologue or epilogue, no segment
- * bookkeeping.  RP particle pairs per thread (1: the library's layout; 2: the alternative with
+ * bookkeeping.  RP particle pairs per thread (1, or 2 with
  * twice the FMAs per shared load), U records unrolled.  Throughput is reported in particle-points
  * per second and as algorithmic TFLOP/s (18 + 6 NI flops per particle-point, the library's count)
  * against the FFMA peak given on the command line.
