@@ -949,8 +949,8 @@ static int fill_data(lgb_ctx *c, int n, const double *coords, const double *valu
    40 us); else the smallest of 32, 64 and 128 that holds a mean cell, so that units of sparse cells cost no
    idle warps (1M particles of a mixture over 970,000 cells: 32 threads 3.0 ms per launch, 128 threads
    23.5 ms).  From 128 particles per cell on, 128 or 256 by the warps their units keep busy, where
-   two particles per thread cost 1.8 of one (563 per cell, 16.8M particles: 256 22.6 ms, 128 25.1 ms;
-   144 per cell, 2M particles: 128 3.4 ms, 256 4.7 ms).
+   two particles per thread cost 1.94 of one (a pass of 16.8M particles at 563 per cell: 256 99.7 ms, 128 102.4 ms;
+   2M at 144: 128 28.8 ms, 256 40.5 ms; 4M at 134: 16.5, 22.6).
    Gather kernels: the cost of a capacity C = 64m (m = 1, 2) is, per work unit, one warp-equivalent of
    block staging plus its active warps plus a third of a warp for each warp left without particles
    (it still stages and occupies the SM). */
@@ -983,7 +983,7 @@ static int choose_chunk(lgb_ctx *c)
       for (i = 0; i < nc; i++) {
         n = cnt[i + 1] - cnt[i];
         c1 += 4.0 * (double)(n / 128) + unit_warps((int)(n % 128));
-        c2 += 7.2 * (double)(n / 256) + (n % 256 > 128 ? 7.2 : unit_warps((int)(n % 256)));
+        c2 += 7.75 * (double)(n / 256) + (n % 256 > 128 ? 7.75 : unit_warps((int)(n % 256)));
       }
       if (c1 <= c2) cap = 128;
     }
