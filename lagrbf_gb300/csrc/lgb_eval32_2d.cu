@@ -9,14 +9,17 @@ static int launch32r(const EvalParams &P, int grid, cudaStream_t s)
 {
   static bool attr = false;
   const int nbuf = 1;
+  /* at least a warp: the kernel's block table takes 3^DIM threads and its votes whole warps (units of 32
+     particles are cut for the record kernel, which other fields of the same particles do not take) */
+  const int threads = P.chunk_cap / R < 32 ? 32 : P.chunk_cap / R;
   /* staging buffer(s) + per-thread running sums of the R*NEN*FP per-patch partial sums */
-  size_t smem = ((size_t)nbuf * P.budget + (size_t)(R * (1 << DIM) * FP + 1) * (P.chunk_cap / R)) * sizeof(float);
+  size_t smem = ((size_t)nbuf * P.budget + (size_t)(R * (1 << DIM) * FP + 1) * threads) * sizeof(float);
   if (!attr) {
     size_t smax = ((size_t)nbuf * P.budget + (size_t)(R * (1 << DIM) * FP + 1) * (LGB_CHUNK_MAX / R)) * sizeof(float);
     cudaFuncSetAttribute(k_eval<float, DIM, FP, R, KER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
     attr = true;
   }
-  k_eval<float, DIM, FP, R, KER><<<grid, P.chunk_cap / R, smem, s>>>(P);
+  k_eval<float, DIM, FP, R, KER><<<grid, threads, smem, s>>>(P);
   return (int)cudaGetLastError();
 }
 

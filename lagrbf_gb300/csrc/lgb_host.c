@@ -951,7 +951,7 @@ static int fill_data(lgb_ctx *c, int n, const double *coords, const double *valu
    23.5 ms).  From 128 particles per cell on, 128 or 256 by the warps their units keep busy, where
    two particles per thread cost 1.94 of one (a pass of 16.8M particles at 563 per cell: 256 99.7 ms, 128 102.4 ms;
    2M at 144: 128 28.8 ms, 256 40.5 ms; 4M at 134: 16.5, 22.6).
-   Gather kernels: the cost of a capacity C = 64m (m = 1, 2) is, per work unit, one warp-equivalent of
+   Gather kernels: the cost of a capacity C = 64m (m = 1 to 4) is, per work unit, one warp-equivalent of
    block staging plus its active warps plus a third of a warp for each warp left without particles
    (it still stages and occupies the SM). */
 static double unit_warps(int n); /* warps that a unit of n <= 128 particles keeps busy */
@@ -987,7 +987,7 @@ static int choose_chunk(lgb_ctx *c)
       }
       if (c1 <= c2) cap = 128;
     }
-    if (!d->rec32 && cap < 64) cap = 64; /* gather kernel, or no data yet */
+    if ((!d->rec32 || d->F > d->g.dim) && cap < 64) cap = 64; /* gather kernel for some fields, or no data yet */
     if (cap < 128) threads = cap;
   } else if (fx) {
     for (cap = 128; cap > 32; cap /= 2) {
