@@ -487,7 +487,9 @@ static int read_options(lgb_ctx *c)
   d->fixed = g->kernel == LGB_KERNEL_WENDLAND_C2 ? 1 : g->kernel == LGB_KERNEL_GAUSSIAN ? 2 : 0;
   for (i = 0; i < dim; i++)
     if (!(g->eps_r * g->h[i] < 32.0) || !(g->eps_w * g->h[i] < 32.0)) d->fixed = 0;
-  if (g->wr > 8) d->fixed = 0; /* the weights of the support nodes add up to less than 2^7 */
+  /* the weights of the support nodes must add up to less than 2^7 (in 3D 103 at a radius of 7 spacings, 126 at
+     7.5, 153 at 8) */
+  if (g->wr > 7) d->fixed = 0;
   d->F = 0;
   opt_int("n_interpolation_fields", &d->F);
   if (d->F < 0) return set_error(LAGRBF_ERR_ARG_OUTOFRANGE, "n_interpolation_fields must be >= 0");
