@@ -16,7 +16,10 @@ extern "C" int lgb_build_records_2d(const EvalParams *P, int force, int grid, vo
    table (lgb_eval_tune.h: stage count and size), FP64 48 KB. */
 #define BUDGET32 7680
 #include "lgb_eval_tune.h"
-#define BUDGET32_TMA LGB_TMA_BUDGET_TUNED /* floats per staging round of the record kernel */
+#define BUDGET32_TMA LGB_TMA_BUDGET_TUNED /* floats per staging round of the record kernel, units of 128 */
+#ifndef EVR_NB
+#define EVR_NB LGB_EVR_NB_TUNED
+#endif
 #define BUDGET64 6144
 /* Polls of a bounded mbarrier wait of the evaluation kernel before it reports a timeout. */
 #define EVAL_POLL_LIMIT (1 << 22)
@@ -53,7 +56,7 @@ static int tma_budget(void)
   static int b = -1;
   if (b < 0) {
     const char *e = getenv("LAGRBF_TMA_BUDGET");
-    b = (e && atoi(e) >= 1024) ? (atoi(e) / 4) * 4 : BUDGET32_TMA;
+    b = (e && atoi(e) >= 256) ? atoi(e) : BUDGET32_TMA;
   }
   return b;
 }
@@ -101,7 +104,7 @@ extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int ou
     if (d->prec == LGB_PREC_FP32) {
       const int stage = (d->rec32 && f == 0 && fp == g.dim && d->rec_fp == g.dim) ? 1 : 0;
       /* the ring grows with the unit, and for more than 128 threads so that their streams find segments in it */
-      P.budget = !stage ? BUDGET32 : d->unit_threads > 128 ? d->unit_threads * 32 : tma_budget() * d->chunk_cap / 128;
+      P.budget = stage ? lgb_stage_floats(tma_budget(), EVR_NB, d->unit_threads, d->chunk_cap) : BUDGET32;
       rc = (g.dim == 3) ? lgb_eval32_launch_3d(&P, fp, ker, stage, grid, stream)
                         : lgb_eval32_launch_2d(&P, fp, ker, stage, grid, stream);
     } else if (d->fixed) {

@@ -44,6 +44,20 @@ enum { LGB_VF_NONE = 0, LGB_VF_ROTATION = 1, LGB_VF_CELLULAR = 2, LGB_VF_ABC = 3
    coordinate floats and 2 floats per (field, involved patch), padded to 16 bytes. */
 #define LGB_NVSEG(dim) ((dim) == 3 ? 28 : 9)
 #define LGB_REC2_LEN(dim, ninv, fp) (((2 * (dim) + 2 * (ninv) * (fp) + 3) / 4) * 4)
+/* Floats of one of the record kernel's ring stages for work units of `cap` particles on `threads` threads, from the
+   floats `base` of a unit of 128: in proportion to the unit, and 32 per thread for more than 128 threads.  A multiple of
+   4 (stages start on 16 bytes, as bulk copies must); all stages together within 2^15 floats (of 227 KB per CTA) and each
+   within 2^14 (the planner's division by the record length is exact up to there), and not fewer than the final sums
+   of the shares take in the drained ring (3 fields of 8 bytes per thread; a record has 32 floats at most). */
+static inline int lgb_stage_floats(long long base, int stages, int threads, int cap)
+{
+  const long long least = 6 * threads / stages + 4;
+  long long most = (1 << 15) / stages, b = threads > 128 ? 32LL * threads : base * cap / 128;
+  if (most > 1 << 14) most = 1 << 14;
+  if (b < least) b = least;
+  if (b > most) b = most;
+  return (int)(b / 4 * 4);
+}
 /* Patch-size classes of the set-up / solve launches: class c holds the patches of up to
    32 * 2^c points (the last class every larger one); LGB_FACT_T is the CTA size of a class without a
    measured entry.  A class with CTAs of T threads keeps 1024 / T of them in flight per SM. */
