@@ -2,23 +2,21 @@
  * lgb_eval32_2d.cu -- FP32-evaluation instantiations of the PU evaluation kernel (lgb_eval.cuh), 2D.
  */
 #include "lgb_evalrec.cuh"
+#include "lgb_optin.cuh"
 #include <stdlib.h>
 
 template <int DIM, int FP, int KER, int R>
 static int launch32r(const EvalParams &P, int grid, cudaStream_t s)
 {
-  static bool attr = false;
+  static unsigned long long opted = 0;
   const int nbuf = 1;
   /* at least a warp: the kernel's block table takes 3^DIM threads and its votes whole warps (units of 32
      particles are cut for the record kernel, which other fields of the same particles do not take) */
   const int threads = P.chunk_cap / R < 32 ? 32 : P.chunk_cap / R;
   /* staging buffer(s) + per-thread running sums of the R*NEN*FP per-patch partial sums */
   size_t smem = ((size_t)nbuf * P.budget + (size_t)(R * (1 << DIM) * FP + 1) * threads) * sizeof(float);
-  if (!attr) {
-    size_t smax = ((size_t)nbuf * P.budget + (size_t)(R * (1 << DIM) * FP + 1) * (LGB_CHUNK_MAX / R)) * sizeof(float);
-    cudaFuncSetAttribute(k_eval<float, DIM, FP, R, KER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smax);
-    attr = true;
-  }
+  const size_t smax = ((size_t)nbuf * P.budget + (size_t)(R * (1 << DIM) * FP + 1) * (LGB_CHUNK_MAX / R)) * sizeof(float);
+  if (const int rc = lgb_opt_in(k_eval<float, DIM, FP, R, KER>, (int)smax, &opted)) return rc;
   k_eval<float, DIM, FP, R, KER><<<grid, threads, smem, s>>>(P);
   return (int)cudaGetLastError();
 }
@@ -35,18 +33,10 @@ static int launch32(const EvalParams &P, int grid, cudaStream_t s)
 template <int DIM, int KER, int RM>
 static int launch_rec(const EvalParams &P, int grid, cudaStream_t s)
 {
-  /* the attribute is set once to the device's largest opt-in size (threads racing on it all set the
-     same value; a per-call size could shrink it under another thread's launch) */
-  static int attr = 0;
+  /* opted in once to the device's largest size (a per-call size could shrink it under another thread's launch) */
+  static unsigned long long opted = 0;
   const size_t smem = ((size_t)EVR_NB * P.budget + (size_t)(RM == 2 ? 2 * EVR_T : P.threads) * 10) * sizeof(float);
-  if (!attr) {
-    int dev = 0, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    cudaFuncSetAttribute(k_eval_rec<DIM, DIM, KER, RM>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         optin - 8192);
-    attr = 1;
-  }
+  if (const int rc = lgb_opt_in(k_eval_rec<DIM, DIM, KER, RM>, 227 * 1024 - 8192, &opted)) return rc;
   k_eval_rec<DIM, DIM, KER, RM><<<grid, P.threads, smem, s>>>(P);
   return (int)cudaGetLastError();
 }

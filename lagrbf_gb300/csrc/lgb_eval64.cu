@@ -3,6 +3,7 @@
  * lgb_op_eval and the FP64 PU-weights kernel.
  */
 #include "lgb_eval.cuh"
+#include "lgb_optin.cuh"
 #include <string.h>
 #include <stdlib.h>
 
@@ -27,13 +28,9 @@ extern "C" int lgb_build_records_2d(const EvalParams *P, int force, int grid, vo
 template <int DIM, int FP>
 static int launch64(const EvalParams &P, int grid, cudaStream_t s)
 {
-  static bool attr = false;
+  static unsigned long long opted = 0;
   size_t smem = (size_t)P.budget * sizeof(double);
-  if (!attr) {
-    cudaFuncSetAttribute(k_eval<double, DIM, FP, 1, KER_GENERIC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
-    attr = true;
-  }
+  if (const int rc = lgb_opt_in(k_eval<double, DIM, FP, 1, KER_GENERIC>, (int)smem, &opted)) return rc;
   k_eval<double, DIM, FP, 1, KER_GENERIC><<<grid, P.chunk_cap, smem, s>>>(P);
   return (int)cudaGetLastError();
 }

@@ -26,6 +26,7 @@
  */
 #include "lgb_common.cuh"
 #include "lgb_fx.cuh"
+#include "lgb_optin.cuh"
 
 #define CHOL_NB 16 /* columns per Cholesky panel */
 
@@ -1142,12 +1143,10 @@ extern "C" int lgb_op_factor(lgb_dev *d, void *stream)
     cudaStream_t s = (cudaStream_t)stream;
     switch (d->cls_threads[c]) {
     case 0: {
-      static int attr = 0; /* threads racing on it all set the same value */
-      if (!attr) {
-        cudaFuncSetAttribute(k_factor_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(BlkShared));
-        cudaFuncSetAttribute(k_solve_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(FxSolveShared));
-        attr = 1;
-      }
+      static unsigned long long opted_f = 0, opted_s = 0;
+      int rc = lgb_opt_in(k_factor_blk, (int)sizeof(BlkShared), &opted_f);
+      if (!rc) rc = lgb_opt_in(k_solve_blk, (int)sizeof(FxSolveShared), &opted_s);
+      if (rc) return rc;
       k_factor_blk<<<d->cls_grid[c], BLK_NT, sizeof(BlkShared), s>>>(P, &d->ctrl->next_c[c]);
       if (P.keep) {
         FactorParams Q = P;
