@@ -42,10 +42,17 @@ struct FxeShared {
   int seg_v[28], seg_p0[28], seg_n[28], seg_base[28], nseg;
   int vs, pp;                /* planner cursor */
   int cell, pbeg, pn, blk, wsum;
-  double scale[4];           /* units of the field sums, NaN where a coefficient is not finite */
   unsigned long long den[FXE_T];
   unsigned long long w[8][FXE_T]; /* phiW of the corners */
 };
+
+/* x 2^e for |e| <= 2044, in two steps (one factor has exponents from -1022 to 1023); NaN for e = LGB_CEXP_NAN. */
+__device__ __forceinline__ double fxe_scale(double x, int e)
+{
+  if (e == LGB_CEXP_NAN) return __hiloint2double(0x7ff80000, 0);
+  const int a = e >> 1, b = e - a;
+  return x * __hiloint2double((1023 + a) << 20, 0) * __hiloint2double((1023 + b) << 20, 0);
+}
 
 template <int DIM, int KER>
 __device__ __forceinline__ long long fxe_phi(long long dx, long long dy, long long dz)
@@ -173,11 +180,10 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
   }
   __syncthreads();
   if (tid < FP) { /* the fields' common exponents */
-    int e = -900;
+    int e = LGB_CEXP_ZERO;
     for (int k = 0; k < NEN; k++)
       if (S.setup[k]) e = max(e, P.cexp[(size_t)S.node[k] * P.F + P.f0 + tid]);
     S.exps[tid] = e;
-    S.scale[tid] = e < 2000 ? __hiloint2double((1023 + 8 - fxe_fine<KER> + e) << 20, 0) : __hiloint2double(0x7ff80000, 0);
   }
   if (tid == 32) {
     int nb = 0;
@@ -277,7 +283,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
         for (int t = tid; t < n * FP; t += FXE_T) {
           const int p = t / FP, f = t - p * FP;
           int2 v = make_int2(0, 0);
-          if (on && S.exps[f] < 2000) {
+          if (on && S.exps[f] != LGB_CEXP_NAN) {
             const double c = P.c64[(size_t)(pos + p) * P.F + P.f0 + f];
             /* c 2^(56 - e) by the exponent field; what is too small for it is below half a unit */
             const int up = 56 - S.exps[f], hi = __double2hiint(c), ec = (hi >> 20) & 2047;
@@ -312,13 +318,13 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
   __syncthreads();
   if (active && sh == 0 && idx < pn) {
     double *o = P.out + (size_t)pid * P.out_stride;
-    const double den = (double)(long long)S.den[idx], sc = den > 0.0 ? __hiloint2double((1023 - ws) << 20, 0) / den : 0.0;
+    const double den = (double)(long long)S.den[idx], sc = den > 0.0 ? __hiloint2double((1023 + 8 - fxe_fine<KER> - ws) << 20, 0) / den : 0.0;
 #pragma unroll
     for (int f = 0; f < FP; f++) {
       for (int k = 1; k < ns; k++)
         for (int h = 0; h < 2; h++) val[f][h] += red[(((k - 1) * FP + f) * 2 + h) * (FXE_T / 2) + idx];
       val[f][1] += val[f][0] >> 32;
-      o[f] = fma((double)val[f][1], 4294967296.0, (double)(val[f][0] & 0xffffffffll)) * sc * S.scale[f];
+      o[f] = fxe_scale(fma((double)val[f][1], 4294967296.0, (double)(val[f][0] & 0xffffffffll)) * sc, S.exps[f]);
     }
   }
   /* algorithmic work of this unit (the same count as the FP64 kernel) */

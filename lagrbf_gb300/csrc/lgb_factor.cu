@@ -669,7 +669,7 @@ __device__ __forceinline__ void blk_mma(float (&c)[4], const unsigned (&a)[4], u
 __device__ __forceinline__ void fx_pack(FxSolveShared &S, int q, int lane, double v)
 {
   const unsigned top = __reduce_max_sync(0xffffffffu, (unsigned)__double2hiint(v) & 0x7fffffffu) >> 20;
-  const int e = max((int)top - 1022, -900); /* |v| < 2^e */
+  const int e = max((int)top - 1022, -966); /* |v| < 2^e, and both factors below are normal */
   const double up = __hiloint2double((1023 + 56 - e) << 20, 0);
   S.yq[q][lane] = fx_split(top == 2047 ? 0 : __double2ll_rn(v * up));
   if (lane == 0) S.ysc[q] = top == 2047 ? __hiloint2double(0x7ff80000, 0) : __hiloint2double((1023 - 56 + e) << 20, 0);

@@ -80,6 +80,8 @@ static inline LGB_HD int lgb_patch_class(int m)
   while (c < LGB_NCLS - 1 && m > (32 << c)) c++;
   return c;
 }
+/* The exponent kept with a patch's coefficients: |c| < 2^e; zero (or subnormal) throughout, not finite. */
+#define LGB_CEXP_ZERO (-1022)
 #define LGB_CEXP_NAN 0x7fffffff
 /* 8-byte elements of the blocked kernel's stored factor of m points (layout in lgb_factor.cu). */
 static inline LGB_HD long long lgb_fx_size(int m)
