@@ -13,10 +13,12 @@
  * centre cell in two halves, so that a record carries at most four patches), staging per data point
  *     { x, y, [z] } and { X_k[j, f] } for every field f and involved corner patch k
  * in shared memory: coordinates in units of the support radius relative to the evaluating cell's
- * origin, coefficients relative to a power of two above the largest one of the field in the cell's
- * patches, both fixed point, the coefficients as {hi, lo}.  Every lane reads the same record
+ * origin, coefficients relative to a power of two above the largest one of the patch and field,
+ * both fixed point, the coefficients as {hi, lo}.  Every lane reads the same record
  * (broadcast).  A segment's per-patch sums are exact 64-bit sums; after FXE_RUN records they
- * are folded, still as whole numbers, into the particle's field sums with the PU weights.  Units of up to 64
+ * are folded, still as whole numbers, into the particle's field sums with the PU weights, in units that go by the patches
+ * with a share in the particle's value: a patch of large coefficients (points that nearly coincide) costs no bits where its
+ * weight is zero or small.  Units of up to 64
  * particles divide the runs of records among their warps (a cell of 20 particles would otherwise leave three of
  * four warps idle); whole numbers make the result independent of it, and so of the unit's other particles.
  * The PU weights are fixed point too, divided at the end by an exact sum over the support nodes, which the
@@ -29,6 +31,7 @@
 #define FXE_T 128       /* threads */
 #define FXE_RUN 32      /* records between folds (32 products below 2^56 stay within 63 bits) */
 #define FXE_BUDGET 24576 /* bytes of staged records */
+#define FXE_SHARE 8     /* PU weights from 2^-8 of the support sum on set the units of the fields */
 
 /* Bytes of a record: coordinates (3D: padded to 32), coefficients. */
 __host__ __device__ constexpr int fxe_len(int dim, int ninv, int fp)
@@ -37,7 +40,9 @@ __host__ __device__ constexpr int fxe_len(int dim, int ninv, int fp)
 }
 
 struct FxeShared {
-  int cnt[27], first[27], node[8], setup[8], exps[4];
+  int exps[8][4];            /* exponents above the corner patches' coefficients, by field */
+  int cnt[27], first[27], node[8], setup[8];
+  int bad;                   /* fields with a coefficient that is not finite */
   long long off[27][3];      /* neighbour cell's origin relative to the cell's */
   int seg_v[28], seg_p0[28], seg_n[28], seg_base[28], nseg;
   int vs, pp;                /* planner cursor */
@@ -46,10 +51,9 @@ struct FxeShared {
   unsigned long long w[8][FXE_T]; /* phiW of the corners */
 };
 
-/* x 2^e for |e| <= 2044, in two steps (one factor has exponents from -1022 to 1023); NaN for e = LGB_CEXP_NAN. */
+/* x 2^e for |e| <= 2044, in two steps (one factor has exponents from -1022 to 1023). */
 __device__ __forceinline__ double fxe_scale(double x, int e)
 {
-  if (e == LGB_CEXP_NAN) return __hiloint2double(0x7ff80000, 0);
   const int a = e >> 1, b = e - a;
   return x * __hiloint2double((1023 + a) << 20, 0) * __hiloint2double((1023 + b) << 20, 0);
 }
@@ -80,11 +84,13 @@ __device__ __forceinline__ long long fxe_weigh(long long s, unsigned long long w
 
 /* The runs of FXE_RUN records of a piece (n records of NI patches at rec) whose number is the share's (run: of
    the round, so far), for the lane's particle: the per-patch sums of a run are folded into val, two words per
-   field, with the PU weights w[corner * FXE_T].  A run's fold is a whole number that does not depend on which
+   field, with the PU weights w[corner * FXE_T], which carry the patches' exponents ex[corner][field] relative to the
+   particle's: w 2^(ex - ef) stays below bit 63.  A run's fold is a whole number that does not depend on which
    share does it, and so neither does their sum. */
 template <int DIM, int FP, int KER, int NI>
 __device__ __forceinline__ void fxe_segment(const unsigned char *rec, int n, int sh, int ns, int &run, long long px, long long py,
-                                            long long pz, unsigned mask, const unsigned long long *w, int ws, long long (&val)[FP][2])
+                                            long long pz, unsigned mask, const unsigned long long *w, const int (*ex)[4],
+                                            const int (&ef)[FP], int ws, long long (&val)[FP][2])
 {
   constexpr int LEN = fxe_len(DIM, NI, FP), HEAD = DIM == 3 ? 32 : 16;
   for (int p0 = 0; p0 < n; p0 += FXE_RUN, run++) {
@@ -117,11 +123,13 @@ __device__ __forceinline__ void fxe_segment(const unsigned char *rec, int n, int
     unsigned m = mask;
 #pragma unroll
     for (int j = 0; j < NI; j++) {
-      const unsigned long long wk = w[(__ffs(m) - 1) * FXE_T] << ws;
+      const int k = __ffs(m) - 1;
+      const unsigned long long wk = w[k * FXE_T];
       m &= m - 1;
 #pragma unroll
       for (int f = 0; f < FP; f++) {
-        const long long v = fxe_weigh<KER>(fx_sum(hh[j * FP + f], hl[j * FP + f]), wk);
+        const int up = ws - ef[f] + ex[k][f];
+        const long long v = fxe_weigh<KER>(fx_sum(hh[j * FP + f], hl[j * FP + f]), up >= 0 ? wk << min(up, 63) : wk >> min(-up, 63));
         val[f][0] += v & 0xffffffffll;
         val[f][1] += v >> 32;
       }
@@ -160,6 +168,7 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
       S.pbeg = P.pstart[c] + b0;
       S.pn = b1 - b0;
       S.wsum = 0;
+      S.bad = 0;
       S.vs = 0;
       S.pp = 0;
     }
@@ -179,11 +188,10 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     S.off[o][d] = fx_coord(g.eps_r, (g.O[d] + g.h[d] * (cc[d] + a)) - org[d]);
   }
   __syncthreads();
-  if (tid < FP) { /* the fields' common exponents */
-    int e = LGB_CEXP_ZERO;
-    for (int k = 0; k < NEN; k++)
-      if (S.setup[k]) e = max(e, P.cexp[(size_t)S.node[k] * P.F + P.f0 + tid]);
-    S.exps[tid] = e;
+  if (tid < NEN * FP) {
+    const int k = tid / FP, f = tid - k * FP, e = S.setup[k] ? P.cexp[(size_t)S.node[k] * P.F + P.f0 + f] : LGB_CEXP_ZERO;
+    S.exps[k][f] = e == LGB_CEXP_NAN ? LGB_CEXP_ZERO : e;
+    if (e == LGB_CEXP_NAN) atomicOr(&S.bad, 1 << f);
   }
   if (tid == 32) {
     int nb = 0;
@@ -237,11 +245,20 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
     if (idx >= pn) wloc = 0;
   }
   __syncthreads();
-  /* the support sum in bit 62; the division by it comes last */
-  unsigned long long wmax = 1;
+  /* The support sum in bit 62 (the division by it comes last), and the fields' exponents: the largest ex of the patches
+     with a share of 2^-8 or more in the sum, and large enough that w 2^(ex - ef) stays below bit 63 for the others. */
+  const int ws = __clzll((long long)max(S.den[idx], 1ull)) - 1;
+  int ef[FP];
 #pragma unroll
-  for (int k = 0; k < NEN; k++) wmax = max(wmax, S.w[k][idx]);
-  const int ws = __clzll((long long)max(S.den[idx], wmax)) - 1;
+  for (int f = 0; f < FP; f++) ef[f] = LGB_CEXP_ZERO;
+#pragma unroll
+  for (int k = 0; k < NEN; k++) {
+    const unsigned long long wk = S.w[k][idx];
+    const int over = max(wk ? __clzll((long long)wk) - ws - 1 : INT_MAX, 0); /* bits of the sum above the weight's */
+#pragma unroll
+    for (int f = 0; f < FP; f++)
+      if (wk) ef[f] = max(ef[f], S.exps[k][f] - (over <= FXE_SHARE ? 0 : over));
+  }
 
   long long val[FP][2];
 #pragma unroll
@@ -283,10 +300,10 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
         for (int t = tid; t < n * FP; t += FXE_T) {
           const int p = t / FP, f = t - p * FP;
           int2 v = make_int2(0, 0);
-          if (on && S.exps[f] != LGB_CEXP_NAN) {
+          if (on && !((S.bad >> f) & 1)) {
             const double c = P.c64[(size_t)(pos + p) * P.F + P.f0 + f];
             /* c 2^(56 - e) by the exponent field; what is too small for it is below half a unit */
-            const int up = 56 - S.exps[f], hi = __double2hiint(c), ec = (hi >> 20) & 2047;
+            const int up = 56 - S.exps[k][f], hi = __double2hiint(c), ec = (hi >> 20) & 2047;
             if (ec > 0 && ec + up > 0) v = fx_split(__double2ll_rn(__hiloint2double(hi + (up << 20), __double2loint(c))));
           }
           *reinterpret_cast<int2 *>(dst + (size_t)p * len + (DIM == 3 ? 32 : 16) + 8 * (j * FP + f)) = v;
@@ -301,9 +318,9 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
         const unsigned char *rec = smem_raw + S.seg_base[i];
         const unsigned long long *w = &S.w[0][idx];
         switch (__popc(mask)) {
-        case 1: fxe_segment<DIM, FP, KER, 1>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, ws, val); break;
-        case 2: fxe_segment<DIM, FP, KER, 2>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, ws, val); break;
-        default: fxe_segment<DIM, FP, KER, 4>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, ws, val); break;
+        case 1: fxe_segment<DIM, FP, KER, 1>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, S.exps, ef, ws, val); break;
+        case 2: fxe_segment<DIM, FP, KER, 2>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, S.exps, ef, ws, val); break;
+        default: fxe_segment<DIM, FP, KER, 4>(rec, n, sh, ns, run, pq[0], pq[1], pq[2], mask, w, S.exps, ef, ws, val); break;
         }
       }
     __syncthreads();
@@ -324,7 +341,8 @@ __global__ void __launch_bounds__(FXE_T, 4) k_eval_fx(EvalParams P)
       for (int k = 1; k < ns; k++)
         for (int h = 0; h < 2; h++) val[f][h] += red[(((k - 1) * FP + f) * 2 + h) * (FXE_T / 2) + idx];
       val[f][1] += val[f][0] >> 32;
-      o[f] = fxe_scale(fma((double)val[f][1], 4294967296.0, (double)(val[f][0] & 0xffffffffll)) * sc, S.exps[f]);
+      const double v = fma((double)val[f][1], 4294967296.0, (double)(val[f][0] & 0xffffffffll)) * sc;
+      o[f] = (S.bad >> f) & 1 ? __hiloint2double(0x7ff80000, 0) : fxe_scale(v, ef[f]);
     }
   }
   /* algorithmic work of this unit (the same count as the FP64 kernel) */
