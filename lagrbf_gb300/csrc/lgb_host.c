@@ -431,7 +431,7 @@ static int read_options(lgb_ctx *c)
   lgb_dev *d = &c->d;
   lgb_geom *g = &d->g;
   int dim = 0, n[3] = {0, 0, 0}, nn, k, i;
-  double O[3] = {0, 0, 0}, L[3] = {1, 1, 1}, overlap = 1.0, shape = 1.0, box = 0.0, radius;
+  double O[3] = {0, 0, 0}, L[3] = {1, 1, 1}, overlap = 1.0, shape = 1.0, box = 0.0, radius, diag;
   char buf[64];
   memset(g, 0, sizeof(*g));
   if (!opt_int("pu_mesh_dim", &dim)) return set_error(LAGRBF_ERR_ARG_WRONG, "option -pu_mesh_dim not provided");
@@ -490,6 +490,11 @@ static int read_options(lgb_ctx *c)
   /* the weights of the support nodes must add up to less than 2^7 (in 3D 103 at a radius of 7 spacings, 126 at
      7.5, 153 at 8) */
   if (g->wr > 7) d->fixed = 0;
+  /* and near a cell's middle, farthest from the nodes, one must be above 2^-6: they are whole numbers of 2^-56, and where
+     the supports hardly reach each other their sum would hold few bits (FP64's error of the largest weight is as much at
+     1 - r = 1/4) */
+  for (i = 0, diag = 0.0; i < dim; i++) diag += g->h[i] * g->h[i];
+  if (!(0.5 * sqrt(diag) * g->eps_w <= 0.75)) d->fixed = 0;
   d->F = 0;
   opt_int("n_interpolation_fields", &d->F);
   if (d->F < 0) return set_error(LAGRBF_ERR_ARG_OUTOFRANGE, "n_interpolation_fields must be >= 0");
