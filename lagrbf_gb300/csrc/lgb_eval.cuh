@@ -62,6 +62,7 @@ struct EvalParams {
   int withhold_copies;    /* test hook: arm the staging barriers but issue no copy         */
   const long long *xq;    /* [nd*dim] eps (x - own cell's origin) in fixed point, cell order */
   const int *cexp;        /* [nnodes*F] exponents above the patches' coefficients             */
+  int phi_bits;           /* log2, rounded up, of the largest kernel value around a cell */
   unsigned char *cdirty;  /* cells whose record blocks must be rebuilt (set by the work-list compaction) */
 };
 

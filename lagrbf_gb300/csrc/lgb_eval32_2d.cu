@@ -28,14 +28,14 @@ static int launch32(const EvalParams &P, int grid, cudaStream_t s)
   return launch32r<DIM, FP, KER, 2>(P, grid, s);
 }
 
-/* The record-streamed kernel: EVR_NB stages of P.budget floats, the PU weights and the shares' support
-   sums (10 words per thread). */
+/* The record-streamed kernel: EVR_NB stages of P.budget floats; per particle the PU weights (8 words) and marks of its sums
+   (1), per thread the shares' support sums (2). */
 template <int DIM, int KER, int RM>
 static int launch_rec(const EvalParams &P, int grid, cudaStream_t s)
 {
   /* opted in once to the device's largest size (a per-call size could shrink it under another thread's launch) */
   static unsigned long long opted = 0;
-  const size_t smem = ((size_t)EVR_NB * P.budget + (size_t)(RM == 2 ? 2 * EVR_T : P.threads) * 10) * sizeof(float);
+  const size_t smem = ((size_t)EVR_NB * P.budget + (size_t)(RM == 2 ? 2 * EVR_T * 10 : P.threads * 11)) * sizeof(float);
   if (const int rc = lgb_opt_in(k_eval_rec<DIM, DIM, KER, RM>, 227 * 1024 - 8192, &opted)) return rc;
   k_eval_rec<DIM, DIM, KER, RM><<<grid, P.threads, smem, s>>>(P);
   return (int)cudaGetLastError();

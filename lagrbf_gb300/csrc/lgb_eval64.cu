@@ -4,6 +4,7 @@
  */
 #include "lgb_eval.cuh"
 #include "lgb_optin.cuh"
+#include <math.h>
 #include <string.h>
 #include <stdlib.h>
 
@@ -58,6 +59,14 @@ static int tma_budget(void)
   return b;
 }
 
+/* log2, rounded up, of the largest kernel value between the points around a cell: 1, or for the linear and multiquadric
+   kernels at most 1 + eps r, r <= 2 (hx + hy + hz). */
+static int phi_bits(const lgb_geom &g)
+{
+  if (g.kernel != LGB_KERNEL_LINEAR && g.kernel != LGB_KERNEL_MQ) return 0;
+  return (int)ceil(log2(fmin(1.0 + 2.0 * g.eps_r * (g.h[0] + g.h[1] + (g.dim == 3 ? g.h[2] : 0.0)), 1e9)));
+}
+
 /* Evaluate fields [nf_first, nf_first+nf) of the coefficient pool at every live particle and
    write them to out[p*out_stride + (f - nf_first)].  Fields are processed four at a time. */
 extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int out_stride, void *stream)
@@ -97,6 +106,7 @@ extern "C" int lgb_op_eval(lgb_dev *d, int nf_first, int nf, double *out, int ou
     P.withhold_copies = d->eval_withhold;
     P.xq = d->xq;
     P.cexp = d->cexp;
+    P.phi_bits = phi_bits(g);
     int rc;
     if (d->prec == LGB_PREC_FP32) {
       const int stage = (d->rec32 && f == 0 && fp == g.dim && d->rec_fp == g.dim) ? 1 : 0;

@@ -45,3 +45,13 @@ def test_fp64_beyond_the_support_of_large_coefficients(dim, nlat, n, kernel):
     f, g = (fields(dim, nlat, n, kernel, "fp64", near) for near in (False, True))
     assert np.abs(f).max() > 0.1
     assert np.abs(f - g).max() <= 1e-13 * np.abs(f).max()
+
+
+# whole numbers in units of 2^-40 of the largest coefficients in reach or finer, of 64 segments
+@pytest.mark.parametrize("kernel", [2, 5, 6])
+@pytest.mark.parametrize("n", [1, 50, 300])
+@pytest.mark.parametrize("dim,nlat", [(2, 20), (3, 9)])
+def test_fp32_beyond_the_support_of_large_coefficients(dim, nlat, n, kernel):
+    f, g = (fields(dim, nlat, n, kernel, "fp32", near) for near in (False, True))
+    assert np.abs(f).max() > 0.1
+    assert np.abs(f - g).max() <= 1e-9 * np.abs(f).max()
