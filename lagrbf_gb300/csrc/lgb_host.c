@@ -1018,8 +1018,9 @@ static int choose_chunk(lgb_ctx *c)
     }
   }
   free(cnt);
-  if (env && (atoi(env) == 64 || atoi(env) == 128 || (atoi(env) == 256 && !(fx && d->prec != LGB_PREC_FP32)))) {
-    cap = atoi(env);
+  if (env && atoi(env) >= 64 && atoi(env) <= LGB_CHUNK_MAX) { /* in steps of 64; the fixed-point kernel takes 128 at most */
+    cap = atoi(env) / 64 * 64;
+    if (fx && d->prec != LGB_PREC_FP32 && cap > 128) cap = 128;
     threads = cap < 128 ? cap : 128;
   }
   if (cap != d->chunk_cap || threads != d->unit_threads) {
