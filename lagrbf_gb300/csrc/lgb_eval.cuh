@@ -611,30 +611,6 @@ __device__ __forceinline__ void cell_block(const EvalParams &P, int cell, int *s
   }
 }
 
-/* Builds the staged record blocks of every cell into P.rec32 (FP32, FP fields from field f0), in
-   neighbour-offset order, at P.rec_off[cell].  Runs only when `force` or when the preceding
-   factorisation launch set up or solved at least one patch (device-side count), so the launch can
-   sit in the captured step graph. */
-template <int DIM, int FP>
-__global__ void __launch_bounds__(128) k_build_records(EvalParams P, int force)
-{
-  constexpr int NOFF = EGeo<DIM>::NOFF;
-  __shared__ int s_cnt[27], s_first[27], s_node[8], s_setup[8];
-  if (!force && P.ctrl->nwork == 0) return;
-  for (int cell = blockIdx.x; cell < P.g.ncells; cell += gridDim.x) {
-    cell_block<DIM>(P, cell, s_cnt, s_first, s_node, s_setup);
-    __syncthreads();
-    float *dst = P.rec32 + P.rec_off[cell];
-    for (int o = 0; o < NOFF; o++) {
-      const int S = erec<float>(epopc(einv_mask(DIM, o)), FP);
-      for (int p = threadIdx.x; p < s_cnt[o]; p += blockDim.x)
-        write_record<float, DIM, FP>(P, o, p, s_first[o] + p, s_node, s_setup, dst + (size_t)p * S);
-      dst += (size_t)s_cnt[o] * S;
-    }
-    __syncthreads();
-  }
-}
-
 /* shared-memory address of a generic pointer (PTX operands) */
 __device__ __forceinline__ unsigned smem_addr(const void *p) { return (unsigned)__cvta_generic_to_shared(p); }
 
