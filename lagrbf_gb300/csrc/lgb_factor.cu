@@ -526,11 +526,14 @@ __global__ void __launch_bounds__(NT) k_factor(FactorParams P)
    2^-56 (lgb_fx.cuh), whose rounding is below that of FP64 from 1/8 on and below what the m rounded
    FP64 subtractions of an entry accumulate:
      - the sums over earlier block columns on the tensor cores: l = sum_i d_i 2^-(9 + 10 i) with six
-       balanced digits |d_i| <= 512, exact in FP16; the products of equal weight i + j <= 5 (21 of 36;
-       the others are below 2^-55 together) accumulate in FP32 and are moved to 64-bit integers every
-       64 columns.  Sums below 2^24 are exact: with row norms <= 1 (Cauchy) those with d_0 stay below
-       2^18 sqrt(64), sum d_1 d_1' <= 64 2^18, and sums of pairs of lower digits are of the order
-       sqrt(64) 2^16.4 (sums of squares on the diagonal 64 2^16.4);
+       balanced digits |d_i| <= 512, exact in FP16; the products of equal weight i + j <= 5 (21 of 36)
+       accumulate in FP32 and are moved to 64-bit integers every 64 columns.  Sums below 2^24 are exact.
+       With row norms <= 1 (Cauchy) those with d_0 stay below 2^18 sqrt(64), and sum d_1 d_1' <= 64 2^18 by
+       itself; sums of pairs of lower digits are of the order sqrt(64) 2^16.4 (sums of squares on the
+       diagonal 64 2^16.4), 2^24 being some 17 standard deviations away: an estimate for digits that are not
+       made to line up, not a bound.  What is left out adds up over the columns: of the products
+       of weight 6 and more the squares d_3^2 on the diagonal have one sign, about m 2^-61.6 together (2^-52.6
+       at 512 columns, 2^-50.6 at 2,048), which FP64's roundings of the m subtractions of a pivot exceed;
      - inside a block column as {hi, lo} integer multiply-adds (fx_mad), in 64-bit sums: |sum hi hi'|
        <= 2^56, |sum hi lo' + lo hi'| <= 2^56 sqrt(32).
    An entry beyond 1 proves a non-positive pivot in its row (a_ii - l_ij^2 < 0): it is clamped for the

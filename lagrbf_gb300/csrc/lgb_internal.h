@@ -14,7 +14,7 @@
  *                   Cholesky factors (only when factors are kept), setup/solved flags
  *   particle swarm  xp[np*dim], fields[np*F], vel[np*dim], x0[np*dim], vadv[7][np*dim] f64,
  *                   cell_p[np], alive[np]; per-stage binning pcount/pstart[ncells+1],
- *                   pfill[ncells], plist[np], chunk_start[ncells+1]
+ *                   plist[np], chunk_start[ncells+1]
  */
 #ifndef LGB_INTERNAL_H
 #define LGB_INTERNAL_H
@@ -35,7 +35,7 @@ enum { LGB_PREC_FP64 = 0, LGB_PREC_FP32 = 1 };
 enum { LGB_VF_NONE = 0, LGB_VF_ROTATION = 1, LGB_VF_CELLULAR = 2, LGB_VF_ABC = 3, LGB_VF_FOURIER = 4 };
 
 /* Largest evaluation work unit (particles of one cell handled by one CTA); the actual capacity
-   (d->chunk_cap, a multiple of 64) is chosen from the particles-per-cell histogram. */
+   (d->chunk_cap, 32 or a multiple of 64) is chosen from the particles-per-cell histogram. */
 #define LGB_CHUNK_MAX 256
 
 /* FP32 record blocks streamed by the evaluation kernel (lgb_evalrec.cuh): per cell, the data

@@ -104,7 +104,7 @@ static long long dataset_bytes(const lagrbf_job_t *j)
   m = 2LL * (1 << j->dim) * ((long long)j->nd / (ncells > 0 ? ncells : 1) + 1) + 16; /* largest patch, generous */
   {
     /* factorisation workspace: (1024 / LGB_FACT_T) patch slots per SM (160 SMs assumed; the blocked
-       factorisation takes two, of less than m * m words each), at most 4 GB, as the context sizes it */
+       factorisation takes two, of 1.3 m * m words (1,700 points; 2.1 at 100) with the factor in them), at most 4 GB, as the context sizes it */
     long long ws = (1024LL / LGB_FACT_T) * 160 * m * m * 8;
     if (ws > (4LL << 30)) ws = 4LL << 30;
     return (long long)j->nd * (long long)(400 + 120 * (1 << j->dim) * j->dim) + nnodes * 64 + ws + (64LL << 20);
