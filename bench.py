@@ -576,7 +576,8 @@ def main():
     ctx.synchronize()
     el64 = allmax(time.perf_counter() - ts)
     value64 = allsum(ctx.stats()["particle_steps"]) / el64
-    # the FP64 evaluation kernel against the FP64 pipe (event-timed launches of one profiled step)
+    # the FP64 path's evaluation kernel, which runs on the integer pipe, against what the FP64 pipe could reach
+    # (event-timed launches of one profiled step)
     ctx.reset_stats()
     ctx.set_profiling(True)
     ctx.advect_resident(t, t + DT)
@@ -586,10 +587,11 @@ def main():
     ctx.set_profiling(False)
     fp64_peak = cf["lagrbf_gpu_fp64_peak_tflops"]()
     e64 = sp64["eval_flops"] / (sp64["eval_ms"] * 1e-3) / 1e12 if sp64["eval_ms"] > 0 else 0.0
-    roofline64 = {"bound": "fp64", "achieved": e64, "peak": fp64_peak, "unit": "TFLOP/s",
+    roofline64 = {"bound": "integer", "achieved": e64, "peak": fp64_peak, "unit": "TFLOP/s",
                   "frac": e64 / fp64_peak if fp64_peak > 0 else None,
-                  "kernel": "k_eval<double,3,3,1,KER_GENERIC> (PU evaluation, FP64 gather path)",
-                  "peak_source": "measured: DFMA-chain probe on this GPU in this run (lagrbf_gpu_fp64_peak_tflops)",
+                  "kernel": "k_eval_fx<3,3,KER_C2> (PU evaluation in 64-bit fixed point)",
+                  "peak_source": "measured: DFMA-chain probe on this GPU in this run (lagrbf_gpu_fp64_peak_tflops); above 1 "
+                                 "because the kernel does not run on that pipe",
                   "per_launch_ms": sp64["eval_ms"] / max(sp64["eval_launches"], 1),
                   "flops_per_launch": sp64["eval_flops"] / max(sp64["eval_launches"], 1)}
     ctx.set_precision(True)
@@ -671,7 +673,7 @@ def main():
             "scaling": "weak", "vs_baseline": None, "dtype": "f32", "data": "synthetic",
             "config": {"workload": "abc3d: %d^3 jittered lattice (%d nodes), ABC flow, %d^3 PU patches, Wendland C2, "
                                    "%d particles/GPU, RK4 dt=%g" % (args.nlat, len(xd), args.npu, args.np, DT),
-                       "eval": "FP32 evaluation, FP64 factorisation and weight normalisation",
+                       "eval": "FP32 evaluation; factorisation and solves with FP64 accuracy (fixed point above 64 points)",
                        "solve_method": {1: "A_KSP (factors resident)", 2: "A_KSP_ASMB (re-factor per solve)"}
                        .get(args.solve_method, str(args.solve_method)),
                        "l2": "inputs larger than L2 (particle state %.1f GB)" % (npart * 8 * 3 * 12 / 1e9),
